@@ -358,6 +358,11 @@ void Solver::step(bool last_in_call) {
 // time_integration.f90, stress.f90 and acceleration.f90 in place.
 void Solver::step_general(bool st) {
     Geom& G = g;
+    if (d.statics_made) {
+        // the stress fields take the statics' place; off the mesh they are zero
+        d.statics_made = false;
+        for (float* f : {d.sd[0], d.sd[1], d.sd[2], d.so[0]}) dev_fill(*this, f, G.nv, 0.f);
+    }
     long long tio = 0;
     auto io = [&](const char* passes, const char* field, FieldView f) {
         long long t0 = clock_us();
@@ -949,6 +954,7 @@ int sord_set_field(sord_handle* h, const char* name, const float* host, size_t n
                 for (int j = 0; j < c[0]; j++)
                     all[(size_t)s.g.idx(s.g.i1core[0] + j, s.g.i1core[1] + k, s.g.i1core[2] + l)] = host[q++];
         SORD_CUDA(cudaMemcpyAsync(dst, all.data(), sizeof(float) * (size_t)s.g.nv, cudaMemcpyHostToDevice, s.stream));
+        if (cell) s.d.statics_made = false;
         SORD_CUDA(cudaStreamSynchronize(s.stream));
     } catch (const std::exception& e) {
         return fail(h, e);

@@ -32,7 +32,11 @@
 // general meshes compute all three.  Each cell's brackets are evaluated
 // once and shared by the cell's gradient and its eight corner nodes'
 // divergence (stencil.cuh: cell_cn_brackets).
+//
+// That is the step in reference order and, on general meshes, in fast
+// arithmetic; rectilinear and terrain meshes take k_modal (modal.cuh) there.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -91,11 +95,7 @@ struct Lay {
     // q, that node's whole force terms from the cell: (fu_x, fu_y, fu_z,
     // fl_x) as float4 group q and (fl_y, fl_z) as float2 in groups 4-5
     static constexpr int NGCR = 6;
-    // ... and on rectilinear and terrain meshes copies each node plane
-    // straight into the ring as raw (u, gam), (v, z) groups: no staging plane
-    static constexpr bool RAWRING = GEOM != GEOM_GENERAL;
-    static constexpr size_t bytes_fm = sizeof(float) * (size_t)(RAWRING ? 0 : RAWSZ) +
-                                       sizeof(float4) * (size_t)(3 * NPL * NGN + NCL * NGCR);
+    static constexpr size_t bytes_fm = sizeof(float) * (size_t)RAWSZ + sizeof(float4) * (size_t)(3 * NPL * NGN + NCL * NGCR);
 };
 // scalar field numbers of the node and cell groups
 __host__ __device__ constexpr int nf_co(int c) { return c == 0 ? 3 : c == 1 ? 7 : 8; }
@@ -202,7 +202,7 @@ struct LayS {
 // at most 15 x 15 nodes), with every PML, boundary and point-source term of
 // the step.
 constexpr int SJ = 16, SK = 16;  // shell tile (cells = threads)
-// FM: the fast arithmetic of k_interior for the support-operator sums.
+// FM (general meshes): the fast arithmetic of k_interior for the support-operator sums.
 template <int GEOM, bool FM>
 __global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_shell(StepArgs A) {
     constexpr int FJ = SJ, FK = SK, FNJ = FJ + 1, FNK = FK + 1, FOJ = FJ - 1, FOK = FK - 1;
@@ -237,7 +237,6 @@ __global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_shell
         tya = A.y1d[K - 1];
         tyb = A.y1d[K];
     }
-    const float hdx = h * (txb - txa), hdy = h * (tyb - tya);
 
     // point injections that fall inside this block (cells / nodes it computes)
     __shared__ Inject lpot[kLocalInject], lmom[kLocalInject], lfrc[kLocalInject];
@@ -359,18 +358,11 @@ __global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_shell
                 for (int n = 0; n < 8; n++)
 #pragma unroll
                     for (int c = 0; c < L::NCOORD; c++) X[3 - L::NCOORD + c][n] = NODE(ns[n], L::CO + c, ni[n]);
-                if (GEOM == GEOM_TERRAIN) {
-                    terrain_brackets_0(hdy, X[2], B[0]);
-                    terrain_brackets_1(hdx, X[2], B[1]);
 #pragma unroll
-                    for (int t = 0; t < 8; t++) B[2][t] = A.brh.bnc[2][t];
-                } else {
+                for (int a = 0; a < 3; a++) {
+                    brackets_nc(X, a, B[a]);
 #pragma unroll
-                    for (int a = 0; a < 3; a++) {
-                        brackets_nc(X, a, B[a]);
-#pragma unroll
-                        for (int t = 0; t < 8; t++) B[a][t] = h * B[a][t];
-                    }
+                    for (int t = 0; t < 8; t++) B[a][t] = h * B[a][t];
                 }
 #pragma unroll
                 for (int a = 0; a < L::NDIR; a++)
@@ -776,23 +768,19 @@ __device__ __forceinline__ void zero_cell_fr(float4* sC, int tid, int ncl) {
 
 // Interior kernel: tiles of 31 x 7 nodes from (A.jf, A.kf), planes A.lf0..A.lf1,
 // strictly inside the non-PML region, with no PML or boundary terms.
-// FM (fast arithmetic): fused multiply-adds, brackets scaled by h once per
-// cell, divergence brackets taken as the negated gradient brackets and, on
-// terrain meshes, the closed-form brackets of stencil.cuh; equal to the
-// reference-order kernel in exact arithmetic, not bit for bit.
+// FM (fast arithmetic, general meshes; k_modal has the others): fused
+// multiply-adds, brackets scaled by h once per cell, divergence brackets
+// taken as the negated gradient brackets; equal to the reference-order
+// kernel in exact arithmetic, not bit for bit.
 template <int GEOM, bool FASTK, bool FM>
 __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(StepArgs A) {
     using L = Lay<GEOM>;
     constexpr int NGN = L::NGN, NGC = L::NGC, NDIR = L::NDIR;
     extern __shared__ float4 sm4[];
-    // fast arithmetic on rectilinear and terrain meshes: the ring holds the
-    // raw (u, gam) and (v, z) of each node, copied in by cp.async, and a
-    // cell forms w and the hourglass input of its corners from them
-    constexpr bool RR = FM && L::RAWRING;
+    static_assert(!FM || GEOM == GEOM_GENERAL, "k_modal takes the other meshes in fast arithmetic");
     float* sR = reinterpret_cast<float*>(sm4);  // [RAWF][NPL] staged plane
-    float4* sN = sm4 + (RR ? 0 : L::RAWSZ / 4);  // [3 slots][NGN][NPL]
-    float4* sC = sN + 3 * NGN * NPL;            // [2 slots][NGC][NCL]; fast arithmetic [NGCF][NCL]
-    constexpr int NQ = L::NQ, NGCF = L::NGCF;
+    float4* sN = sm4 + L::RAWSZ / 4;            // [3 slots][NGN][NPL]
+    float4* sC = sN + 3 * NGN * NPL;            // [2 slots][NGC][NCL]; fast arithmetic [NGCR][NCL]
 #define RAW(f, i) sR[(f) * NPL + (i)]
     const Geom& g = A.g;
     const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + FJ * ty;
@@ -817,8 +805,6 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
         tya = A.y1d[K - 1];
         tyb = A.y1d[K];
     }
-    // fast arithmetic on terrain meshes: the bracket spacings times h
-    const float hdx = h * (txb - txa), hdy = h * (tyb - tya);
 
     // point injections that fall inside this block (cells / nodes it computes)
     __shared__ Inject lpot[kLocalInject], lmom[kLocalInject], lfrc[kLocalInject];
@@ -843,25 +829,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
                 const int nj = n % FNJ, nk = n / FNJ;
                 const int j = j0 - 1 + nj, k = k0 - 1 + nk;
                 const bool ok = j <= g.nm[0] && k <= g.nm[1] && l >= 1 && l <= g.nm[2];
-                if (RR) {
-                    // ring slot of plane l: group 0 (u, gam), group 1 (v, z)
-                    float* d0 = reinterpret_cast<float*>(sN + (l % 3) * (NGN * NPL) + n);
-                    float* d1 = reinterpret_cast<float*>(sN + (l % 3) * (NGN * NPL) + NPL + n);
-                    if (ok) {
-                        const long long q = g.idx(j, k, l);
-#pragma unroll
-                        for (int c = 0; c < 3; c++) {
-                            cp_async4(d0 + c, A.uin[c] + q);
-                            cp_async4(d1 + c, A.vin[c] + q);
-                        }
-                        cp_async4(d0 + 3, A.gam + q);
-                        if (GEOM == GEOM_TERRAIN) cp_async4(d1 + 3, A.x[2] + q);
-                        else d1[3] = 0.f;
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < 4; c++) { d0[c] = 0.f; d1[c] = 0.f; }
-                    }
-                } else if (ok) {
+                if (ok) {
                     const long long q = g.idx(j, k, l);
 #pragma unroll
                     for (int c = 0; c < 3; c++) {
@@ -950,12 +918,9 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
     } while (0)
 
     // ---------------------------------------------------------------- cell phase
-    constexpr bool CARRY = FM && GEOM != GEOM_GENERAL;
-    float4 ca[4], cb[4];  // plane l+1 corners of the last cell computed, for plane l+1's cell
     // fast arithmetic: the terms of this thread's own cell for its own node
     // column (reader q = 0) stay in registers for the node phase
     float ownu[3] = {0.f, 0.f, 0.f}, ownl[3] = {0.f, 0.f, 0.f};
-    int carry_l = -1000;  // the plane of that cell
     auto cells = [&](int l, auto fast_tag) {
         constexpr bool F = decltype(fast_tag)::value;
         const int cs = FM ? 0 : l & 1;
@@ -973,37 +938,15 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
             return;
         }
         const long long q = g.idx(J, K, l);
-        // corner values by corner id n = dj + 2 dk + 4 dl (node planes l, l+1);
-        // fast arithmetic keeps the plane l+1 corners for the next plane's cell
+        // corner values by corner id n = dj + 2 dk + 4 dl (node planes l, l+1)
         float Wc[3][8], Hc[3][8], X0[8], X1[8], X2[8];
         {
             const float4* p0 = sN + (l % 3) * (NGN * NPL) + (tx + FNJ * ty);
             const float4* p1 = sN + ((l + 1) % 3) * (NGN * NPL) + (tx + FNJ * ty);
-            const bool reuse = CARRY && carry_l == l - 1;
 #pragma unroll
             for (int n = 0; n < 8; n++) {
                 const float4* p = ((n >> 2) ? p1 : p0) + (n & 1) + FNJ * ((n >> 1) & 1);
-                float4 a, b;
-                if (CARRY && n < 4 && reuse) {
-                    a = ca[n];
-                    b = cb[n];
-                } else {
-                    a = p[0];
-                    b = p[NPL];
-                    if constexpr (RR) {
-                        // raw (u, gam), (v, z) -> (w, z), (hourglass input, 0):
-                        // w1 = u + gam * v (time_integration.f90:36) and
-                        // hg1 u + dt hg2 v (acceleration.f90:141)
-                        const float4 u = a, v = b;
-                        a = make_float4(fmaf(u.w, v.x, u.x), fmaf(u.w, v.y, u.y), fmaf(u.w, v.z, u.z), v.w);
-                        b = make_float4(fmaf(A.dh2, v.x, A.hg1 * u.x), fmaf(A.dh2, v.y, A.hg1 * u.y),
-                                        fmaf(A.dh2, v.z, A.hg1 * u.z), 0.f);
-                    }
-                }
-                if (CARRY && n >= 4) {
-                    ca[n - 4] = a;
-                    cb[n - 4] = b;
-                }
+                const float4 a = p[0], b = p[NPL];
                 Wc[0][n] = a.x; Wc[1][n] = a.y; Wc[2][n] = a.z;
                 Hc[0][n] = b.x; Hc[1][n] = b.y; Hc[2][n] = b.z;
                 if (GEOM == GEOM_TERRAIN) {
@@ -1016,32 +959,19 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
                     X2[n] = p[2 * NPL].x;
                 }
             }
-            if (CARRY) carry_l = l;
         }
         // support-operator brackets; directions 0 and 1 in the two lanes
         float B[3][8];
         float cnb[NDIR > 0 ? NDIR : 1][8];
         if constexpr (FM) {
             // brackets scaled by h; divergence brackets = negated gradient brackets
-            if (GEOM == GEOM_RECT) {
+            brackets_nc_g<float>(X1, X2, B[0]);
+            brackets_nc_g<float>(X2, X0, B[1]);
+            brackets_nc_g<float>(X0, X1, B[2]);
 #pragma unroll
-                for (int a = 0; a < 3; a++)
+            for (int a = 0; a < 3; a++)
 #pragma unroll
-                    for (int t = 0; t < 8; t++) B[a][t] = A.brh.bnc[a][t];
-            } else if (GEOM == GEOM_TERRAIN) {
-                terrain_brackets_0(hdy, X2, B[0]);
-                terrain_brackets_1(hdx, X2, B[1]);
-#pragma unroll
-                for (int t = 0; t < 8; t++) B[2][t] = A.brh.bnc[2][t];
-            } else {
-                brackets_nc_g<float>(X1, X2, B[0]);
-                brackets_nc_g<float>(X2, X0, B[1]);
-                brackets_nc_g<float>(X0, X1, B[2]);
-#pragma unroll
-                for (int a = 0; a < 3; a++)
-#pragma unroll
-                    for (int t = 0; t < 8; t++) B[a][t] = h * B[a][t];
-            }
+                for (int t = 0; t < 8; t++) B[a][t] = h * B[a][t];
 #pragma unroll
             for (int a = 0; a < NDIR; a++)
 #pragma unroll
@@ -1643,56 +1573,12 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
 #pragma unroll
         for (int i = 0; i < 3; i++) fc[i] = fl[i];
         if (!finish) return;
-        if constexpr (RR) {
-            // this node's raw u, v from ring slot l
-            const float4* pn = sN + (l % 3) * (NGN * NPL) + (tx + 1) + FNJ * (ty + 1);
-            const float4 a = pn[0], b = pn[NPL];
-            const float uvl[6] = {a.x, a.y, a.z, b.x, b.y, b.z};
-            finish_node<FM>(A, g.idx(jn, kn, l), jn, kn, l, fu, cur[4], uvl, dt, st_a, st_v, st_u);
-        } else {
-            finish_node<FM>(A, g.idx(jn, kn, l), jn, kn, l, fu, cur[4], uv, dt, st_a, st_v, st_u);
-        }
+        finish_node<FM>(A, g.idx(jn, kn, l), jn, kn, l, fu, cur[4], uv, dt, st_a, st_v, st_u);
     };
 
     // ---------------------------------------------------------------- stream
     // ring: planes L0-1, L0, L0+1; staged: L0+2 in flight
     constexpr std::integral_constant<bool, FASTK> path{};
-    if constexpr (RR) {
-        // raw ring: planes L0-1, L0, L0+1 straight into their slots; plane
-        // l + 3 goes into slot l once cells(l) and nodes(l) are done with it
-#pragma unroll 1
-        for (int p = -1; p <= 1; p++) fetch(L0 + p);
-        cp_async_wait_all();
-        __syncthreads();
-        stat_load(L0 - 1, cur);
-        cells(L0 - 1, path);
-        __syncthreads();  // cell plane L0-1 complete: its terms for node L0
-        nodes_fm(L0 - 1, false);
-        __syncthreads();  // one cell slot: read before cells(L0) overwrites it; slot L0-1 free
-        fetch(L0 + 2);
-        stat_load(L0, cur);
-#pragma unroll 1
-        for (int l = L0; l <= L1; l++) {
-            cells(l, path);
-            float nxt[5];
-            stat_load(l + 1, nxt);
-            cp_async_wait_all();
-            __syncthreads();  // cell plane l complete, plane l+2 landed
-            nodes_fm(l, true);
-            __syncthreads();  // cell plane and ring slot l free
-            fetch(l + 3);
-#pragma unroll
-            for (int i = 0; i < 5; i++) cur[i] = nxt[i];
-        }
-        cp_async_wait_all();
-        if (A.stats) {
-            bmax(A.red + 0, st_a);
-            bmax(A.red + 1, st_v);
-            bmax(A.red + 2, st_u);
-            bmax(A.red + 3, st_w);
-        }
-        return;
-    }
 #pragma unroll 1
     for (int p = -1; p <= 1; p++) {
         fetch(L0 + p);
@@ -1741,6 +1627,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
 #undef HVALS
 }
 
+#include "modal.cuh"
 #include "slab.cuh"
 
 // A region of shell items made by one push_box call: boxes of 15 x 15
@@ -1760,6 +1647,7 @@ struct BoxRegion {
 // masked 15 x 15 node boxes for the shell kernel.  Boxes and tiles partition
 // the nodes, so every node, and every PML memory, is updated once.
 struct FusedPlan {
+    int arith = 0;                              // the arithmetic it was made for
     int jf = 0, jend = -1, kf = 0, kend = -1;   // interior rectangle (inclusive)
     int nbx = 0, nby = 0;                       // interior tiles
     int lf0 = 0, lf1 = -1;                      // interior node planes (inclusive)
@@ -1804,9 +1692,12 @@ void fused_free(Solver& s) {
 // Planes per block.  Each block streams its column through the planes, so
 // a small mesh is cut into shorter plane ranges until both kernels have
 // about kWaveBlocks blocks per SM; a range starts with a prologue of about
-// two planes, so it is kept at kMinPlanes planes or more.
+// two planes, so it is kept at kMinPlanes planes or more; in fast
+// arithmetic, whose prologue is one cell plane, down to kFewPlanes where a
+// launch would leave SMs without a block.
 static constexpr int kItemPlanes = 96;
 static constexpr int kMinPlanes = 8;
+static constexpr int kFewPlanes = 4;
 static constexpr int kWaveBlocks = 4;
 // planes per item of an interior tile holding a point source (k_shell): a
 // few tile columns only, so short items spread them over the SMs
@@ -1829,9 +1720,17 @@ static void push_box(std::vector<int>& v, int ipl, int j1, int j2, int k1, int k
 }
 
 static FusedPlan& fused_plan(Solver& s) {
-    if (s.fplan) return *s.fplan;
+    if (s.fplan && s.fplan->arith == s.arith) return *s.fplan;
+    if (s.fplan) {
+        // the arithmetic was changed between two steps
+        SORD_CUDA(cudaStreamSynchronize(s.stream));
+        fused_free(s);
+    }
     FusedPlan* P = new FusedPlan();
     s.fplan = P;
+    P->arith = s.arith;
+    // shortest plane range where a launch has less than a block per SM
+    const int few = s.arith ? kFewPlanes : kMinPlanes;
     const Geom& g = s.g;
     // Node c along axis d is interior when it is outside the PML and each
     // adjacent cell is either a real cell outside the PML or a cell outside
@@ -1914,6 +1813,7 @@ static FusedPlan& fused_plan(Solver& s) {
         };
         int ipl = kItemPlanes;
         while (ipl > kMinPlanes && count(ipl) < want) ipl = std::max(kMinPlanes, ipl * 2 / 3);
+        while (ipl > few && count(ipl) < sms) ipl = std::max(few, ipl * 2 / 3);
         iplc[c] = ipl;
     }
     P->regions.clear();
@@ -1932,8 +1832,20 @@ static FusedPlan& fused_plan(Solver& s) {
         P->nbx = (int)div_up(P->jend - P->jf + 1, FOJ);
         P->nby = (int)div_up(P->kend - P->kf + 1, FOK);
         const int planes = P->lf1 - P->lf0 + 1, cols = P->nbx * P->nby;
-        const int nseg = std::max(1, std::min((want + cols - 1) / cols, planes / kMinPlanes));
-        P->segl = (planes + nseg - 1) / nseg;
+        // the split that takes the fewest plane times: rounds of two blocks
+        // per SM, each block its planes and a prologue of about two (aiming
+        // at four blocks per SM instead left a third round of 56 blocks on
+        // 203 x 149 x 97 nodes)
+        double best = 0;
+        for (int n = 1; n <= std::max(1, planes / few); n++) {
+            const int len = (planes + n - 1) / n;
+            const long long blocks = (long long)cols * ((planes + len - 1) / len);
+            const double t = (double)((blocks + 2 * sms - 1) / (2 * sms)) * (len + 2);
+            if (n == 1 || t < best) {
+                best = t;
+                P->segl = len;
+            }
+        }
         P->nseg = (planes + P->segl - 1) / P->segl;
     }
     P->cap = (int)P->base.size() / 6 + 16384;
@@ -1970,34 +1882,78 @@ static void source_tiles(const Solver& s, const FusedPlan& P, const std::vector<
     }
 }
 
-template <int GEOM, bool FASTK>
-static void launch_mode(Solver& s, const StepArgs& A, dim3 grid, cudaStream_t st) {
-    const size_t bytes = FASTK ? (s.arith ? Lay<GEOM>::bytes_fm : Lay<GEOM>::bytes)
-                               : LayS<GEOM, (SJ + 1) * (SK + 1), SJ * SK>::bytes;
-    if (FASTK && s.arith) {
-        smem_limit((const void*)k_interior<GEOM, true, true>, (int)bytes);
-        k_interior<GEOM, true, true><<<grid, dim3(FJ, FK), bytes, st>>>(A);
-    } else if (FASTK) {
-        smem_limit((const void*)k_interior<GEOM, true, false>, (int)bytes);
-        k_interior<GEOM, true, false><<<grid, dim3(FJ, FK), bytes, st>>>(A);
-    } else if (s.arith) {
-        smem_limit((const void*)k_shell<GEOM, true>, (int)bytes);
-        k_shell<GEOM, true><<<grid, dim3(SJ, SK), bytes, st>>>(A);
+template <int GEOM, int MASK>
+static void launch_modal(Solver& s, const StepArgs& A, dim3 grid, cudaStream_t st) {
+    using L = LayM<MASK>;
+    if (A.fold && !A.stats && !A.aout[0] && A.fax < 0) {
+        smem_limit((const void*)k_modal<GEOM, MASK, true>, (int)L::bytes);
+        k_modal<GEOM, MASK, true><<<grid, dim3(L::TJ, L::TK), L::bytes, st>>>(A);
     } else {
-        smem_limit((const void*)k_shell<GEOM, false>, (int)bytes);
-        k_shell<GEOM, false><<<grid, dim3(SJ, SK), bytes, st>>>(A);
+        smem_limit((const void*)k_modal<GEOM, MASK, false>, (int)L::bytes);
+        k_modal<GEOM, MASK, false><<<grid, dim3(L::TJ, L::TK), L::bytes, st>>>(A);
     }
     s.launches++;
     SORD_CUDA(cudaGetLastError());
 }
 
-template <int GEOM, int MASK>
-static void launch_slab_m(Solver& s, const StepArgs& A, unsigned n, cudaStream_t st) {
-    const size_t bytes = LaySl<GEOM>::bytes;
-    smem_limit((const void*)k_slab<GEOM, MASK>, (int)bytes);
-    k_slab<GEOM, MASK><<<dim3(n, 1, 1), dim3(SJ, SK), bytes, st>>>(A);
+template <int GEOM, bool FASTK>
+static void launch_mode(Solver& s, const StepArgs& A, dim3 grid, cudaStream_t st) {
+    // fast arithmetic: k_modal, on general meshes k_interior and k_shell
+    constexpr bool FM = GEOM == GEOM_GENERAL;
+    if constexpr (FASTK) {
+        if (s.arith && !FM) {
+            launch_modal<GEOM, 0>(s, A, grid, st);
+            return;
+        }
+        const size_t bytes = FM && s.arith ? Lay<GEOM>::bytes_fm : Lay<GEOM>::bytes;
+        auto kern = FM && s.arith ? k_interior<GEOM, true, FM> : k_interior<GEOM, true, false>;
+        smem_limit((const void*)kern, (int)bytes);
+        kern<<<grid, dim3(FJ, FK), bytes, st>>>(A);
+    } else {
+        const size_t bytes = LayS<GEOM, (SJ + 1) * (SK + 1), SJ * SK>::bytes;
+        auto kern = FM && s.arith ? k_shell<GEOM, FM> : k_shell<GEOM, false>;
+        smem_limit((const void*)kern, (int)bytes);
+        kern<<<grid, dim3(SJ, SK), bytes, st>>>(A);
+    }
     s.launches++;
     SORD_CUDA(cudaGetLastError());
+}
+
+// Mesh class of the step kernels: in fast arithmetic a rectilinear mesh
+// whose cells are not boxes (a constant shear) takes the general kernels,
+// since k_modal has the axes' own modes only.
+static int step_class(const Solver& s) {
+    if (!s.arith) return s.geom;
+    // k_modal damps every node by dt hg2 in the PML; the reference leaves it
+    // out there for a negative constant
+    if (s.prm.hourglass[1] < 0.f) return GEOM_GENERAL;
+    if (s.geom != GEOM_RECT) return s.geom;
+    for (int a = 0; a < 3; a++) {
+        double m[7] = {}, own = 0;
+        for (int t = 0; t < 8; t++) {
+            const int n = term_corner(t);
+            const int x = (n & 1) * 2 - 1, y = ((n >> 1) & 1) * 2 - 1, z = (n >> 2) * 2 - 1;
+            const int sg[7] = {x, y, z, x * y, y * z, x * z, x * y * z};
+            for (int q = 0; q < 7; q++) m[q] += sg[q] * (double)s.br.bnc[a][t];
+        }
+        own = std::fabs(m[a]);
+        for (int q = 0; q < 7; q++)
+            if (q != a && std::fabs(m[q]) > 1e-6 * own) return GEOM_GENERAL;  // beyond FP32 rounding
+    }
+    return GEOM_RECT;
+}
+
+template <int GEOM, int MASK>
+static void launch_slab_m(Solver& s, const StepArgs& A, unsigned n, cudaStream_t st) {
+    if constexpr (GEOM != GEOM_GENERAL) {
+        launch_modal<GEOM, MASK>(s, A, dim3(n, 1, 1), st);
+    } else {
+        const size_t bytes = LaySl::bytes;
+        smem_limit((const void*)k_slab<MASK>, (int)bytes);
+        k_slab<MASK><<<dim3(n, 1, 1), dim3(SJ, SK), bytes, st>>>(A);
+        s.launches++;
+        SORD_CUDA(cudaGetLastError());
+    }
 }
 
 template <int GEOM>
@@ -2009,16 +1965,31 @@ static void launch_slab_g(Solver& s, const StepArgs& A, int cls, unsigned n, cud
 }
 
 static void launch_slab(Solver& s, const StepArgs& A, int cls, unsigned n, cudaStream_t st) {
-    if (s.geom == GEOM_RECT) launch_slab_g<GEOM_RECT>(s, A, cls, n, st);
-    else if (s.geom == GEOM_TERRAIN) launch_slab_g<GEOM_TERRAIN>(s, A, cls, n, st);
+    const int geom = step_class(s);
+    if (geom == GEOM_RECT) launch_slab_g<GEOM_RECT>(s, A, cls, n, st);
+    else if (geom == GEOM_TERRAIN) launch_slab_g<GEOM_TERRAIN>(s, A, cls, n, st);
     else launch_slab_g<GEOM_GENERAL>(s, A, cls, n, st);
 }
 
 template <bool FASTK>
 static void launch_geom(Solver& s, const StepArgs& A, dim3 grid, cudaStream_t st) {
-    if (s.geom == GEOM_RECT) launch_mode<GEOM_RECT, FASTK>(s, A, grid, st);
-    else if (s.geom == GEOM_TERRAIN) launch_mode<GEOM_TERRAIN, FASTK>(s, A, grid, st);
+    const int geom = FASTK ? step_class(s) : s.geom;
+    if (geom == GEOM_RECT) launch_mode<GEOM_RECT, FASTK>(s, A, grid, st);
+    else if (geom == GEOM_TERRAIN) launch_mode<GEOM_TERRAIN, FASTK>(s, A, grid, st);
     else launch_mode<GEOM_GENERAL, FASTK>(s, A, grid, st);
+}
+
+// The statics of k_modal, laid out anew where they are not valid.
+static const float4* modal_statics(Solver& s) {
+    Device& d = s.d;
+    float4* sta = (float4*)d.sd[0];
+    if (!d.statics_made) {
+        k_statics<<<div_up(std::min(s.g.nv, 148LL * 64 * 256), 256), 256, 0, s.stream>>>(s.g, d.lam, d.mu, d.vc, d.yy, d.mr, sta);
+        s.launches++;
+        SORD_CUDA(cudaGetLastError());
+        d.statics_made = true;
+    }
+    return sta;
 }
 
 void launch_fused(Solver& s, const InjectList& pot, const InjectList& mom, const InjectList& force,
@@ -2034,6 +2005,12 @@ void launch_fused(Solver& s, const InjectList& pot, const InjectList& mom, const
             A.brh.bnc[a][t] = s.g.h * s.br.bnc[a][t];
             A.brh.bcn[a][t] = s.g.h * s.br.bcn[a][t];
         }
+    for (int a = 0; a < 3; a++) {
+        // the bracket's mode along its own axis: the mean over the corners of sign x bracket
+        double m = 0;
+        for (int t = 0; t < 8; t++) m += (((term_corner(t) >> a) & 1) * 2 - 1) * (double)A.brh.bnc[a][t];
+        A.cm[a] = (float)(0.125 * m);
+    }
     A.x1d = d.x1d;
     A.y1d = d.y1d;
     for (int i = 0; i < 3; i++) {
@@ -2049,9 +2026,9 @@ void launch_fused(Solver& s, const InjectList& pot, const InjectList& mom, const
     A.sl = d.slabs;
     for (int i = 0; i < 6; i++) A.gout[i] = d.gb[i];
     A.pot = pot; A.mom = mom; A.force = force;
-    A.hg1 = s.prm.hourglass[0];
-    A.dh2 = s.g.dt * s.prm.hourglass[1];
     A.hourglass = (s.prm.hourglass[0] > 0.f || s.prm.hourglass[1] > 0.f) ? 1 : 0;
+    A.hg1 = A.hourglass ? s.prm.hourglass[0] : 0.f;
+    A.dh2 = A.hourglass ? s.g.dt * s.prm.hourglass[1] : 0.f;
     A.hgvisc = (s.prm.hourglass[1] > 0.f && s.g.npml > 0) ? 1 : 0;
     A.fold = fold ? 1 : 0;
     A.stats = stats ? 1 : 0;
@@ -2069,23 +2046,38 @@ void launch_fused(Solver& s, const InjectList& pot, const InjectList& mom, const
     A.firup = s.g.irup;
     for (int i = 0; i < 3; i++) A.fout[i] = d.w1n[i];
 
+    int ib[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
+    for (const std::vector<Inject>* e : {&hpot, &hmom, &hforce})
+        for (const Inject& x : *e) {
+            const int c[3] = {(int)(x.idx % s.g.sy) + 1, (int)((x.idx / s.g.sy) % s.g.nm[1]) + 1, (int)(x.idx / s.g.sz) + 1};
+            for (int d = 0; d < 3; d++) {
+                ib[d] = std::min(ib[d], c[d]);
+                ib[3 + d] = std::max(ib[3 + d], c[d]);
+            }
+        }
+    for (int d = 0; d < 6; d++) A.ibox[d] = ib[d];
+
     // shell items of this step: the fixed list, plus the interior planes of
     // the interior tiles holding a point source
+    // (k_modal applies point sources itself)
+    const bool modal = s.arith && step_class(s) != GEOM_GENERAL;
+    A.sta = modal ? modal_statics(s) : nullptr;
     std::vector<std::pair<int, int>> src;
-    if (P.nbx > 0) {
+    if (P.nbx > 0 && !modal) {
         source_tiles(s, P, hpot, true, src);
         source_tiles(s, P, hmom, true, src);
         source_tiles(s, P, hforce, false, src);
         std::sort(src.begin(), src.end());
         src.erase(std::unique(src.begin(), src.end()), src.end());
     }
-    // In fast arithmetic the boxes without a point source go to k_slab, by
+    // In fast arithmetic the boxes without a point source go to k_slab (all of
+    // them to k_modal, which applies point sources itself), by
     // class; k_shell takes the rest (the boxes k_shell tests: cells
     // j0-1..j0+14 for potency / moment entries, nodes j0..j0+14 for forces).
     // Upload order: k_shell items, then the k_slab classes.
     const int nbase = (int)P.base.size() / 6;
     std::vector<char> hit(nbase, s.arith ? 0 : 1);
-    if (s.arith) {
+    if (s.arith && !modal) {
         // an entry at (j, k, l) reaches box (j0, k0, L0..L1) when
         // j0 - o <= j <= j0 + 14 (o = 1 for cells), likewise k, and
         // L0 - o <= l <= L1: at most two boxes per axis in each region
@@ -2146,10 +2138,12 @@ void launch_fused(Solver& s, const InjectList& pot, const InjectList& mom, const
     s.prof_begin(KC_FUSED, &e0);
     const bool inner = P.nbx > 0 && P.nby > 0;
     const dim3 igrid(P.nbx, P.nby, P.nseg);
-    // the shell launches: k_shell, then each k_slab class
+    // the shell launches: k_shell and beside it each class.  The classes are
+    // forked before k_shell, whose few source boxes would hold them up
+    // (160 x 144 x 120 perturbed mesh: 640 -> 562 us a step)
     auto shell_launches = [&](cudaStream_t st) {
-        if (nshell > 0) launch_geom<false>(s, A, dim3((unsigned)nshell, 1, 1), st);
         SORD_CUDA(cudaEventRecord(P.cfork, st));
+        if (nshell > 0) launch_geom<false>(s, A, dim3((unsigned)nshell, 1, 1), st);
         int off = nshell;
         for (int m = 0; m < 4; m++) {
             if (nslab[m] == 0) continue;

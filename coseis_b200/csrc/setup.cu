@@ -377,6 +377,7 @@ static void allocate_arrays(Solver& s) {
     long long nv = s.g.nv;
     Device& d = s.d;
     // the volume fields: one zeroed block, each field at a 256-byte boundary
+    // (sd and so in one piece: k_modal's statics use four of them)
     float** const fields[29] = {&d.x[0], &d.x[1], &d.x[2], &d.v[0], &d.v[1], &d.v[2], &d.u[0], &d.u[1], &d.u[2],
                                 &d.w1n[0], &d.w1n[1], &d.w1n[2], &d.sd[0], &d.sd[1], &d.sd[2], &d.so[0], &d.so[1],
                                 &d.so[2], &d.vc, &d.mr, &d.lam, &d.mu, &d.gam, &d.yy, &d.s1, &d.s2,

@@ -1,10 +1,11 @@
-// PML-shell step kernel in fast arithmetic (included by fused.cu).
+// PML-shell step kernel in fast arithmetic on general meshes (included by
+// fused.cu; k_modal has the other meshes).
 //
 // k_slab does, on the node boxes of the PML shell, the same whole step as
 // k_interior in fast arithmetic (fused multiply-adds, h-scaled brackets,
 // divergence brackets as negated gradient brackets, one cell plane in
 // shared memory read once per node plane, hourglass sums combined per
-// reading node in the cell, the upper cell corners carried in registers),
+// reading node in the cell),
 // with the PML terms of the reference added:
 //
 //   cells  strain: the damped direction of a PML cell differentiates v and
@@ -28,27 +29,24 @@
 // point source of the step are left to k_shell.
 #pragma once
 
-template <int GEOM>
 struct LaySl {
+    static constexpr int GEOM = GEOM_GENERAL;
     static constexpr int NPL = (SJ + 1) * (SK + 1);  // 289 nodes per plane
     static constexpr int NCL = SJ * SK;              // 256 cells per plane
-    static constexpr int NCOORD = GEOM == GEOM_RECT ? 0 : GEOM == GEOM_TERRAIN ? 1 : 3;
-    static constexpr int RAWF = 7 + NCOORD;                   // staged plane: u(3) v(3) gam coords
-    static constexpr int RAWSZ = (RAWF * NPL + 3) & ~3;        // floats, float4-aligned end
-    // node groups: (u, coordinate 0), (v, gam), general meshes (coordinates 1, 2)
-    static constexpr int NGN = GEOM == GEOM_GENERAL ? 3 : 2;
+    static constexpr int RAWF = 10;                      // staged plane: u(3) v(3) gam x y z
+    static constexpr int RAWSZ = (RAWF * NPL + 3) & ~3;  // floats, float4-aligned end
+    static constexpr int NGN = 3;                        // node groups: (u, x), (v, gam), (y, z)
     static constexpr int NDIR = Lay<GEOM>::NDIR, NQ = Lay<GEOM>::NQ, NGCF = Lay<GEOM>::NGCF;
     static constexpr size_t bytes = sizeof(float) * (size_t)RAWSZ + sizeof(float4) * (size_t)(3 * NPL * NGN + NCL * NGCF);
 };
 
-template <int GEOM, int MASK>
-__global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_slab(StepArgs A) {
+template <int MASK>
+__global__ void __launch_bounds__(SJ * SK, 1) k_slab(StepArgs A) {
     constexpr int TJ = SJ, TK = SK, TNJ = TJ + 1, TOJ = TJ - 1, TOK = TK - 1;
-    using L = LaySl<GEOM>;
+    using L = LaySl;
     constexpr int NPL_ = L::NPL, NCL_ = L::NCL, NTH_ = TJ * TK;
     constexpr int NGN = L::NGN, NDIR = L::NDIR, NQ = L::NQ, NGCF = L::NGCF;
     constexpr bool DJ = (MASK & 1) != 0, DK = (MASK & 2) != 0, DL = (MASK & 4) != 0;
-    constexpr bool CARRY = GEOM != GEOM_GENERAL;
     extern __shared__ float4 sm4[];
     float* sR = reinterpret_cast<float*>(sm4);  // [RAWF][NPL] staged plane
     float4* sN = sm4 + L::RAWSZ / 4;            // [3 slots][NGN][NPL]
@@ -65,14 +63,6 @@ __global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_slab(
     const bool owncol = J >= j0 && J <= jm && K >= k0 && K <= km;
     const float dt = g.dt;
     float st_a = 0.f, st_v = 0.f, st_u = 0.f, st_w = 0.f;
-    float txa = 0.f, txb = 0.f, tya = 0.f, tyb = 0.f;
-    if (GEOM == GEOM_TERRAIN && cellcol) {
-        txa = A.x1d[J - 1];
-        txb = A.x1d[J];
-        tya = A.y1d[K - 1];
-        tyb = A.y1d[K];
-    }
-    const float hdx = g.h * (txb - txa), hdy = g.h * (tyb - tya);
     // PML slabs of this thread's cell column (near, far) and node column
     const bool cnj = DJ && J <= g.i1pml[0], cfj = DJ && J >= g.i2pml[0] - 1;
     const bool cnk = DK && K <= g.i1pml[1], cfk = DK && K >= g.i2pml[1] - 1;
@@ -96,10 +86,8 @@ __global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_slab(
                         cp_async4(&RAWS(3 + c, n), A.vin[c] + q);
                     }
                     cp_async4(&RAWS(6, n), A.gam + q);
-                    if (GEOM == GEOM_TERRAIN) cp_async4(&RAWS(7, n), A.x[2] + q);
-                    if (GEOM == GEOM_GENERAL)
 #pragma unroll
-                        for (int c = 0; c < 3; c++) cp_async4(&RAWS(7 + c, n), A.x[c] + q);
+                    for (int c = 0; c < 3; c++) cp_async4(&RAWS(7 + c, n), A.x[c] + q);
                 } else {
 #pragma unroll
                     for (int f = 0; f < L::RAWF; f++) RAWS(f, n) = 0.f;
@@ -108,17 +96,16 @@ __global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_slab(
         }
         cp_async_commit();
     };
-    // staged plane -> ring slot: (u, coordinate 0), (v, gam) [, (coordinates 1, 2)]
+    // staged plane -> ring slot: (u, x), (v, gam), (y, z)
     auto store = [&](int slot) {
         float4* dst = sN + slot * (NGN * NPL_);
 #pragma unroll
         for (int r = 0; r < 2; r++) {
             const int n = tid + r * NTH_;
             if (n < NPL_) {
-                const float c0 = L::NCOORD > 0 ? RAWS(7, n) : 0.f;
-                dst[n] = make_float4(RAWS(0, n), RAWS(1, n), RAWS(2, n), c0);
+                dst[n] = make_float4(RAWS(0, n), RAWS(1, n), RAWS(2, n), RAWS(7, n));
                 dst[NPL_ + n] = make_float4(RAWS(3, n), RAWS(4, n), RAWS(5, n), RAWS(6, n));
-                if (NGN > 2) dst[2 * NPL_ + n] = make_float4(L::NCOORD > 2 ? RAWS(8, n) : 0.f, L::NCOORD > 2 ? RAWS(9, n) : 0.f, 0.f, 0.f);
+                dst[2 * NPL_ + n] = make_float4(RAWS(8, n), RAWS(9, n), 0.f, 0.f);
             }
         }
     };
@@ -145,8 +132,6 @@ __global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_slab(
     };
 
     // ---------------------------------------------------------------- cell phase
-    float4 ca[4], cb[4];  // plane l+1 corners of the last cell computed
-    int carry_l = -1000;
     auto cells = [&](int l) {
         const bool valid = cellcol && l >= g.i1cell[2] && l <= g.i2cell[2];
         if (!valid) {
@@ -173,37 +158,17 @@ __global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_slab(
         {
             const float4* p0 = sN + (l % 3) * (NGN * NPL_) + (tx + TNJ * ty);
             const float4* p1 = sN + ((l + 1) % 3) * (NGN * NPL_) + (tx + TNJ * ty);
-            const bool reuse = CARRY && carry_l == l - 1;
 #pragma unroll
             for (int n = 0; n < 8; n++) {
                 const float4* p = ((n >> 2) ? p1 : p0) + (n & 1) + TNJ * ((n >> 1) & 1);
-                float4 a, b;
-                if (CARRY && n < 4 && reuse) {
-                    a = ca[n];
-                    b = cb[n];
-                } else {
-                    a = p[0];
-                    b = p[NPL_];
-                }
-                if (CARRY && n >= 4) {
-                    ca[n - 4] = a;
-                    cb[n - 4] = b;
-                }
+                const float4 a = p[0], b = p[NPL_], c = p[2 * NPL_];
                 Uc[0][n] = a.x; Uc[1][n] = a.y; Uc[2][n] = a.z;
                 Vc[0][n] = b.x; Vc[1][n] = b.y; Vc[2][n] = b.z;
                 Gc[n] = b.w;
-                if (GEOM == GEOM_TERRAIN) {
-                    X0[n] = (n & 1) ? txb : txa;
-                    X1[n] = ((n >> 1) & 1) ? tyb : tya;
-                    X2[n] = a.w;
-                } else if (GEOM == GEOM_GENERAL) {
-                    const float4 c = p[2 * NPL_];
-                    X0[n] = a.w;
-                    X1[n] = c.x;
-                    X2[n] = c.y;
-                }
+                X0[n] = a.w;
+                X1[n] = c.x;
+                X2[n] = c.y;
             }
-            if (CARRY) carry_l = l;
         }
         // region of the cell (stress.f90:18-131, acceleration.f90:136-199)
         const bool cnl = DL && l <= g.i1pml[2], cfl = DL && l >= g.i2pml[2] - 1;
@@ -215,26 +180,14 @@ __global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_slab(
         const bool own = owncol && (l >= L0 || l < g.i1node[2]);
         // brackets scaled by h; divergence brackets = negated gradient brackets
         float B[3][8];
-        float cnb[NDIR > 0 ? NDIR : 1][8];
-        if (GEOM == GEOM_RECT) {
+        float cnb[NDIR][8];
+        brackets_nc_g<float>(X1, X2, B[0]);
+        brackets_nc_g<float>(X2, X0, B[1]);
+        brackets_nc_g<float>(X0, X1, B[2]);
 #pragma unroll
-            for (int a = 0; a < 3; a++)
+        for (int a = 0; a < 3; a++)
 #pragma unroll
-                for (int t = 0; t < 8; t++) B[a][t] = A.brh.bnc[a][t];
-        } else if (GEOM == GEOM_TERRAIN) {
-            terrain_brackets_0(hdy, X2, B[0]);
-            terrain_brackets_1(hdx, X2, B[1]);
-#pragma unroll
-            for (int t = 0; t < 8; t++) B[2][t] = A.brh.bnc[2][t];
-        } else {
-            brackets_nc_g<float>(X1, X2, B[0]);
-            brackets_nc_g<float>(X2, X0, B[1]);
-            brackets_nc_g<float>(X0, X1, B[2]);
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int t = 0; t < 8; t++) B[a][t] = g.h * B[a][t];
-        }
+            for (int t = 0; t < 8; t++) B[a][t] = g.h * B[a][t];
 #pragma unroll
         for (int a = 0; a < NDIR; a++)
 #pragma unroll
@@ -356,17 +309,9 @@ __global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_slab(
             }
             float4* cq = cw + (2 + NQ * q) * NCL_;
             cq[0] = make_float4(yu[0], yu[1], yu[2], yl[0]);
-            if constexpr (NDIR == 3) {
-                const int tu = (q & 1) + 2 + 4 * (q >> 1), tl = (q & 1) + 4 * (q >> 1);
-                cq[NCL_] = make_float4(yl[1], yl[2], cnb[0][tu], cnb[1][tu]);
-                cq[2 * NCL_] = make_float4(cnb[0][tl], cnb[1][tl], cnb[NDIR - 1][tu], cnb[NDIR - 1][tl]);
-            } else if constexpr (NDIR == 2) {
-                const int tu = (q & 1) + 2 + 4 * (q >> 1), tl = (q & 1) + 4 * (q >> 1);
-                cq[NCL_] = make_float4(yl[1], yl[2], cnb[0][tu], cnb[1][tu]);
-                reinterpret_cast<float2*>(sC + (2 + 4 * NQ) * NCL_)[q * NCL_ + tid] = make_float2(cnb[0][tl], cnb[1][tl]);
-            } else {
-                cq[NCL_] = make_float4(yl[1], yl[2], 0.f, 0.f);
-            }
+            const int tu = (q & 1) + 2 + 4 * (q >> 1), tl = (q & 1) + 4 * (q >> 1);
+            cq[NCL_] = make_float4(yl[1], yl[2], cnb[0][tu], cnb[1][tu]);
+            cq[2 * NCL_] = make_float4(cnb[0][tl], cnb[1][tl], cnb[2][tu], cnb[2][tl]);
         }
     };
 
@@ -407,28 +352,8 @@ __global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_slab(
             const float S[6] = {a.x, a.y, a.z, a.w, e.x, e.y};
             const float4* cq = sC + (2 + NQ * q) * NCL_ + ci;
             const float4 y0 = cq[0], y1 = cq[NCL_];
-            const int tu = cj + 2 + 4 * ck, tl = cj + 4 * ck;
-            float Bu[3], Bl[3];
-            if constexpr (NDIR == 3) {
-                const float4 y2 = cq[2 * NCL_];
-                Bu[0] = y1.z;
-                Bu[1] = y1.w;
-                Bl[0] = y2.x;
-                Bl[1] = y2.y;
-                Bu[2] = y2.z;
-                Bl[2] = y2.w;
-            } else if constexpr (NDIR == 2) {
-                const float2 bl = reinterpret_cast<const float2*>(sC + (2 + 4 * NQ) * NCL_)[q * NCL_ + ci];
-                Bu[0] = y1.z;
-                Bu[1] = y1.w;
-                Bl[0] = bl.x;
-                Bl[1] = bl.y;
-            }
-#pragma unroll
-            for (int id = NDIR; id < 3; id++) {
-                Bu[id] = A.brh.bcn[id][tu];
-                Bl[id] = A.brh.bcn[id][tl];
-            }
+            const float4 y2 = cq[2 * NCL_];
+            const float Bu[3] = {y1.z, y1.w, y2.z}, Bl[3] = {y2.x, y2.y, y2.w};
 #pragma unroll
             for (int ic = 0; ic < 3; ic++)
 #pragma unroll

@@ -158,6 +158,11 @@ struct StepArgs {
     int jf, kf, jend, kend, lf0, lf1;
     const int* items;
     float negzero;  // -0.0, the addend of packed products (pair.cuh)
+    // k_modal: the gradient along each axis per unit of the axis's corner
+    // mode (terrain: along z), and the box around the step's point sources
+    float cm[3];
+    int ibox[6];
+    const float4* sta;  // its statics
     // double-node fault: normal axis (0..2, -1 without a fault) and the
     // minus-side node index; nodes of planes firup and firup + 1 keep their
     // force in fout, unscaled, and their v, u are copied by the fold
@@ -172,6 +177,11 @@ __device__ __forceinline__ void cp_async4(float* smem, const float* gmem) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+// wait until all but the last N groups have landed
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 #endif
 
@@ -204,6 +214,10 @@ struct Device {
     // pool, which concurrent handles reuse without synchronising the device
     void* vol = nullptr;
     bool vol_plain = false;
+    // k_modal's statics (per cell lam / V, mu / V, yy and a node's mr, 16
+    // bytes) lie over sd[0..2] and so[0], which only the separate-kernel
+    // step uses: valid until that step runs or a modulus is set
+    bool statics_made = false;
 };
 
 // Fault-plane arrays (dynamic_rupture.f90:22-63), offsets into Device::fp.
