@@ -44,6 +44,7 @@
 #include <vector>
 
 #include "inject.cuh"
+#include "modes.cuh"
 #include "pair.cuh"
 #include "sord.cuh"
 #include "stencil.cuh"
@@ -179,562 +180,7 @@ __device__ __forceinline__ long long slab_idx(const Geom& g, int axis, int t, in
     return a0 + e0 * (a1 + e1 * a2) + (long long)ic * e0 * e1 * e2;
 }
 
-// 4-byte asynchronous global -> shared copy (no register staging).
-
-// Shared-memory layout of the PML-shell kernel: plain per-field planes
-// (node ring: w(3), hourglass input(3), coordinates; cell ring: stress(6),
-// hourglass(12), divergence brackets(8 per direction)).
-template <int GEOM, int NPLS, int NCLS>
-struct LayS {
-    static constexpr int NCOORD = GEOM == GEOM_RECT ? 0 : GEOM == GEOM_TERRAIN ? 1 : 3;
-    static constexpr int RAWF = 7 + NCOORD;   // staged plane: u(3) v(3) gam coords
-    static constexpr int NODEF = 6 + NCOORD;  // ring: w = u + gam v (3), hg1 u + dt hg2 v (3), coords
-    static constexpr int HG = 3;              // first hourglass-input field
-    static constexpr int CO = 6;              // first coordinate field
-    static constexpr int NDIR = GEOM == GEOM_RECT ? 0 : GEOM == GEOM_TERRAIN ? 2 : 3;
-    static constexpr int CELLF = 6 + 12 + 8 * NDIR;  // stress, hourglass, divergence brackets
-    static constexpr size_t bytes = sizeof(float) * (size_t)(NPLS * RAWF + 3 * NPLS * NODEF + 2 * NCLS * CELLF);
-};
-
-
-// PML-shell kernel: 16 x 16 threads per block, each block the node box of
-// one work item of A.items (j0, k0, last j, last k, first and last plane,
-// at most 15 x 15 nodes), with every PML, boundary and point-source term of
-// the step.
 constexpr int SJ = 16, SK = 16;  // shell tile (cells = threads)
-// FM (general meshes): the fast arithmetic of k_interior for the support-operator sums.
-template <int GEOM, bool FM>
-__global__ void __launch_bounds__(SJ * SK, GEOM == GEOM_GENERAL ? 1 : 2) k_shell(StepArgs A) {
-    constexpr int FJ = SJ, FK = SK, FNJ = FJ + 1, FNK = FK + 1, FOJ = FJ - 1, FOK = FK - 1;
-    constexpr int NPL = FNJ * FNK, NCL = FJ * FK, NTH = FJ * FK;
-    (void)FNK;
-    constexpr bool FASTK = false;
-    using L = LayS<GEOM, NPL, NCL>;
-    extern __shared__ float sm[];
-    float* sR = sm;                          // [RAWF][NPL] staged plane
-    float* sN = sR + L::RAWF * NPL;          // [3 slots][NODEF][NPL]
-    float* sC = sN + 3 * L::NODEF * NPL;     // [2 slots][CELLF][NCL]
-#define RAW(f, i) sR[(f) * NPL + (i)]
-#define NODE(slot, f, i) sN[((slot) * L::NODEF + (f)) * NPL + (i)]
-#define CELL(slot, f, i) sC[((slot) * L::CELLF + (f)) * NCL + (i)]
-    const Geom& g = A.g;
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + FJ * ty;
-    const int* it = A.items + 6 * blockIdx.x;
-    const int j0 = it[0], k0 = it[1], jm = it[2], km = it[3], L0 = it[4], L1 = it[5];
-    const int J = j0 - 1 + tx, K = k0 - 1 + ty;      // this thread's cell column
-    const int jn = j0 + tx, kn = k0 + ty;            // this thread's node column
-    const bool outcol = tx < FOJ && ty < FOK && jn <= jm && kn <= km;
-    const bool cellcol = J >= g.i1cell[0] && J <= g.i2cell[0] && K >= g.i1cell[1] && K <= g.i2cell[1];
-    // the cell of node column (J, K) belongs to the block that owns that node
-    const bool owncol = J >= j0 && J <= jm && K >= k0 && K <= km;
-    const float h = g.h, dt = g.dt;
-    float st_a = 0.f, st_v = 0.f, st_u = 0.f, st_w = 0.f;
-    // terrain meshes: this thread's cell column's x (j, j+1) and y (k, k+1)
-    float txa = 0.f, txb = 0.f, tya = 0.f, tyb = 0.f;
-    if (GEOM == GEOM_TERRAIN && cellcol) {
-        txa = A.x1d[J - 1];
-        txb = A.x1d[J];
-        tya = A.y1d[K - 1];
-        tyb = A.y1d[K];
-    }
-
-    // point injections that fall inside this block (cells / nodes it computes)
-    __shared__ Inject lpot[kLocalInject], lmom[kLocalInject], lfrc[kLocalInject];
-    __shared__ int lcnt[3];
-    // A fast-kernel block whose (j, k) box holds a point source of this step
-    // leaves that column to the general kernel (the host lists it there).
-    const int gl1 = FASTK ? 0 : L0 - 1, gl2 = FASTK ? g.nm[2] + 1 : L1;
-    gather_inject(A.pot, lpot, &lcnt[0], g, j0 - 1, j0 + FOJ - 1, k0 - 1, k0 + FOK - 1, gl1, gl2);
-    gather_inject(A.mom, lmom, &lcnt[1], g, j0 - 1, j0 + FOJ - 1, k0 - 1, k0 + FOK - 1, gl1, gl2);
-    gather_inject(A.force, lfrc, &lcnt[2], g, j0, j0 + FOJ - 1, k0, k0 + FOK - 1, FASTK ? gl1 : L0, gl2);
-    __syncthreads();
-    const int npot = lcnt[0], nmom = lcnt[1], nfrc = lcnt[2];
-    if (FASTK && (npot != 0 || nmom != 0 || nfrc != 0)) return;
-
-    // ---------------------------------------------------------------- loads
-    // stage node plane l (u, v, gam, coordinates) into sR asynchronously
-    auto fetch = [&](int l) {
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            const int n = tid + r * NTH;
-            if (n < NPL) {
-                const int nj = n % FNJ, nk = n / FNJ;
-                const int j = j0 - 1 + nj, k = k0 - 1 + nk;
-                const bool ok = j <= g.nm[0] && k <= g.nm[1] && l >= 1 && l <= g.nm[2];
-                if (ok) {
-                    const long long q = g.idx(j, k, l);
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        cp_async4(&RAW(c, n), A.uin[c] + q);
-                        cp_async4(&RAW(3 + c, n), A.vin[c] + q);
-                    }
-                    cp_async4(&RAW(6, n), A.gam + q);
-                    if (GEOM == GEOM_TERRAIN) cp_async4(&RAW(7, n), A.x[2] + q);
-                    if (GEOM == GEOM_GENERAL)
-#pragma unroll
-                        for (int c = 0; c < 3; c++) cp_async4(&RAW(7 + c, n), A.x[c] + q);
-                } else {
-#pragma unroll
-                    for (int f = 0; f < L::RAWF; f++) RAW(f, n) = 0.f;
-                }
-            }
-        }
-        cp_async_commit();
-    };
-    // staged plane -> ring slot: w1 = u + gam * v (time_integration.f90:36)
-    // and the hourglass input hg1 u + dt hg2 v (acceleration.f90:141)
-    auto store = [&](int slot) {
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            const int n = tid + r * NTH;
-            if (n < NPL) {
-                const float gm = RAW(6, n);
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    const float u = RAW(c, n), v = RAW(3 + c, n);
-                    NODE(slot, c, n) = FM ? fmaf(gm, v, u) : u + gm * v;
-                    NODE(slot, L::HG + c, n) = FM ? fmaf(A.dh2, v, A.hg1 * u) : A.hg1 * u + A.dh2 * v;
-                }
-#pragma unroll
-                for (int f = 0; f < L::NCOORD; f++) NODE(slot, L::CO + f, n) = RAW(7 + f, n);
-            }
-        }
-    };
-
-    // per-plane statics of this thread's cell (lam, mu, 1/V, yy) and node
-    // (mass ratio), loaded one plane ahead of their use
-    float cur[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    auto stat_load = [&](int l, float* o) {
-        const bool cv = cellcol && l >= g.i1cell[2] && l <= g.i2cell[2];
-        const long long qc = cv ? g.idx(J, K, l) : 0;
-        o[0] = cv ? A.lam[qc] : 0.f;
-        o[1] = cv ? A.mu[qc] : 0.f;
-        o[2] = cv ? A.vc[qc] : 0.f;
-        o[3] = cv ? A.yy[qc] : 0.f;
-        const bool nv = outcol && l >= g.i1node[2] && l <= g.i2node[2];
-        o[4] = nv ? A.mr[g.idx(jn, kn, l)] : 0.f;
-    };
-    // this thread's node u, v (for the update and statistics), one plane ahead
-    float uv[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    auto uv_load = [&](int l, float* o) {
-        const bool nv = outcol && l >= g.i1node[2] && l <= g.i2node[2];
-        const long long q = nv ? g.idx(jn, kn, l) : 0;
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            o[c] = nv ? A.uin[c][q] : 0.f;
-            o[3 + c] = nv ? A.vin[c][q] : 0.f;
-        }
-    };
-
-    // ---------------------------------------------------------------- cell phase
-    auto cells = [&](int l, auto fast_tag) {
-        constexpr bool F = decltype(fast_tag)::value;
-        const int cs = l & 1;
-        const bool valid = F || (cellcol && l >= g.i1cell[2] && l <= g.i2cell[2]);
-        float ed[3] = {0.f, 0.f, 0.f}, eo[3] = {0.f, 0.f, 0.f};
-        float he[12];
-#pragma unroll
-        for (int i = 0; i < 12; i++) he[i] = 0.f;
-        float cnb[L::NDIR > 0 ? L::NDIR : 1][8];
-        if (valid) {
-            const long long q = g.idx(J, K, l);
-            const int s0 = l % 3, s1 = (l + 1) % 3;
-            int ni[8], ns[8];
-#pragma unroll
-            for (int n = 0; n < 8; n++) {
-                ni[n] = (tx + (n & 1)) + FNJ * (ty + ((n >> 1) & 1));
-                ns[n] = (n >> 2) ? s1 : s0;
-            }
-            float B[3][8];
-            if (GEOM == GEOM_RECT) {
-#pragma unroll
-                for (int a = 0; a < 3; a++)
-#pragma unroll
-                    for (int t = 0; t < 8; t++) B[a][t] = FM ? A.brh.bnc[a][t] : A.br.bnc[a][t];
-            } else if constexpr (FM) {
-                // brackets scaled by h; divergence brackets = negated gradient brackets
-                float X[3][8];
-#pragma unroll
-                for (int n = 0; n < 8; n++)
-#pragma unroll
-                    for (int c = 0; c < L::NCOORD; c++) X[3 - L::NCOORD + c][n] = NODE(ns[n], L::CO + c, ni[n]);
-#pragma unroll
-                for (int a = 0; a < 3; a++) {
-                    brackets_nc(X, a, B[a]);
-#pragma unroll
-                    for (int t = 0; t < 8; t++) B[a][t] = h * B[a][t];
-                }
-#pragma unroll
-                for (int a = 0; a < L::NDIR; a++)
-#pragma unroll
-                    for (int t = 0; t < 8; t++) cnb[a][t] = -B[a][cn_of_nc(t)];
-            } else {
-                float X[3][8];
-                if (GEOM == GEOM_TERRAIN) {
-                    const float xa = txa, xb = txb, ya = tya, yb = tyb;
-#pragma unroll
-                    for (int n = 0; n < 8; n++) {
-                        X[0][n] = (n & 1) ? xb : xa;
-                        X[1][n] = ((n >> 1) & 1) ? yb : ya;
-                        X[2][n] = NODE(ns[n], L::CO, ni[n]);
-                    }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 3; c++)
-#pragma unroll
-                        for (int n = 0; n < 8; n++) X[c][n] = NODE(ns[n], L::CO + c, ni[n]);
-                }
-#pragma unroll
-                for (int a = 0; a < L::NDIR; a++) {
-                    brackets_nc(X, a, B[a]);
-                    cell_cn_brackets(X, a, B[a], cnb[a]);
-                }
-                if (GEOM == GEOM_TERRAIN)
-#pragma unroll
-                    for (int t = 0; t < 8; t++) B[2][t] = A.br.bnc[2][t];
-            }
-            // a cell plane below the first node plane is a halo of a partitioned run;
-            // the part takes it (the PML g memory of that halo cell advances here)
-            const bool own = owncol && (l >= L0 || l < g.i1node[2]);
-            if constexpr (F) {
-                // strain of an interior cell: gradients of w = u + gam v
-#pragma unroll
-                for (int ic = 0; ic < 3; ic++) {
-                    float W[8];
-#pragma unroll
-                    for (int t = 0; t < 8; t++) {
-                        const int n = term_corner(t);
-                        W[t] = NODE(ns[n], ic, ni[n]);
-                    }
-#pragma unroll
-                    for (int iid = 0; iid < 3; iid++) {
-                        const int id = (ic + iid + 1) % 3;
-                        const float s = stencil8(W, B[id], h);
-                        if (ic == id) ed[ic] = s;
-                        else if (ic < id) eo[3 - ic - id] = 0.5f * s;
-                        else eo[3 - ic - id] = eo[3 - ic - id] + 0.5f * s;
-                    }
-                }
-            } else {
-                // region of the cell (stress.f90:141-248)
-                bool nearS[3], farS[3], anyS = false;
-                const int cc[3] = {J, K, l};
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    nearS[d] = cc[d] <= g.i1pml[d];
-                    farS[d] = cc[d] >= g.i2pml[d] - 1;
-                    anyS = anyS || nearS[d] || farS[d];
-                }
-                // PML cells that are not elastic-hourglass cells carry the
-                // viscous hourglass values dt hg2 yy hourglass_nc(v) in the
-                // hourglass slots (acceleration.f90:164-183)
-                bool inEc = true;
-#pragma unroll
-                for (int d = 0; d < 3; d++) inEc = inEc && cc[d] >= g.i1pml[d] && cc[d] <= g.i2pml[d] - 1;
-                const bool visc = A.hourglass && A.hgvisc && anyS && !inEc;
-                const float yv = A.dh2 * cur[3];
-#pragma unroll
-                for (int ic = 0; ic < 3; ic++) {
-                    float W[8], U[8], V[8];
-#pragma unroll
-                    for (int t = 0; t < 8; t++) {
-                        const int n = term_corner(t);
-                        W[t] = NODE(ns[n], ic, ni[n]);
-                        U[t] = 0.f;
-                        V[t] = 0.f;
-                    }
-                    if (anyS) {
-#pragma unroll
-                        for (int t = 0; t < 8; t++) {
-                            const int n = term_corner(t);
-                            const long long qn = g.idx(J + (n & 1), K + ((n >> 1) & 1), l + (n >> 2));
-                            U[t] = A.uin[ic][qn];
-                            V[t] = A.vin[ic][qn];
-                        }
-                    }
-                    if (visc) {
-                        float Vc[8], Vh[8];
-#pragma unroll
-                        for (int t = 0; t < 8; t++) Vc[term_corner(t)] = V[t];
-#pragma unroll
-                        for (int t = 0; t < 8; t++) Vh[t] = Vc[hg_corner(t)];
-#pragma unroll
-                        for (int iq = 0; iq < 4; iq++) he[3 * iq + ic] = yv * hg_sum(Vh, iq);
-                    }
-#pragma unroll
-                    for (int iid = 0; iid < 3; iid++) {
-                        const int id = (ic + iid + 1) % 3;
-                        float s;
-                        if (nearS[id] || farS[id]) {
-                            const float raw = FM ? dot8(V, B[id]) : stencil8(V, B[id], h);
-                            s = raw;
-                            const int c = cc[id];
-                            if (nearS[id]) {
-                                const int p = c + g.nnoff[id];
-                                const long long gi = slab_idx(g, id, A.sl.tg[id], c - g.i1cell[id], J, K, l, ic);
-                                s = A.pmlc[3 * g.npml + p - 1] * raw + A.pmlc[2 * g.npml + p - 1] * A.sl.g[id][gi];
-                                if (own) A.gout[id][gi] = s;
-                            }
-                            if (farS[id]) {
-                                const int p = g.nn[id] - c - g.nnoff[id];
-                                const long long gi = slab_idx(g, id, A.sl.tg[3 + id], g.i2cell[id] - c, J, K, l, ic);
-                                s = A.pmlc[3 * g.npml + p - 1] * raw + A.pmlc[2 * g.npml + p - 1] * A.sl.g[3 + id][gi];
-                                if (own) A.gout[3 + id][gi] = s;
-                            }
-                        } else if (anyS) {
-                            s = FM ? dot8(U, B[id]) : stencil8(U, B[id], h);
-                        } else {
-                            s = FM ? dot8(W, B[id]) : stencil8(W, B[id], h);
-                        }
-                        if (ic == id) ed[ic] = s;
-                        else if (ic < id) eo[3 - ic - id] = 0.5f * s;
-                        else eo[3 - ic - id] = eo[3 - ic - id] + 0.5f * s;
-                    }
-                }
-                apply_inject(lpot, npot, A.pot, q, ed, eo);
-            }
-            {
-                const float lm = cur[0], m2 = 2.0f * cur[1];
-                const float s1v = lm * (ed[0] + ed[1] + ed[2]);
-#pragma unroll
-                for (int i = 0; i < 3; i++) { ed[i] = m2 * ed[i] + s1v; eo[i] = m2 * eo[i]; }
-            }
-            if constexpr (!F) apply_inject(lmom, nmom, A.mom, q, ed, eo);
-            {
-                const float r = cur[2];
-#pragma unroll
-                for (int i = 0; i < 3; i++) { ed[i] = ed[i] * r; eo[i] = eo[i] * r; }
-            }
-            if (A.stats && own)
-                st_w = fmaxn(st_w, (ed[0] * ed[0] + ed[1] * ed[1] + ed[2] * ed[2]) + 2.0f * (eo[0] * eo[0] + eo[1] * eo[1] + eo[2] * eo[2]));
-            // elastic hourglass cell values (acceleration.f90:141-156)
-            if (A.hourglass) {
-                bool inE = true;
-                if constexpr (!F) {
-                    const int cc[3] = {J, K, l};
-#pragma unroll
-                    for (int d = 0; d < 3; d++) inE = inE && cc[d] >= g.i1pml[d] && cc[d] <= g.i2pml[d] - 1;
-                }
-                if (inE) {
-                    const float y = cur[3];
-#pragma unroll
-                    for (int ic = 0; ic < 3; ic++) {
-                        float W2[8];
-#pragma unroll
-                        for (int t = 0; t < 8; t++) {
-                            const int n = hg_corner(t);
-                            W2[t] = NODE(ns[n], L::HG + ic, ni[n]);
-                        }
-#pragma unroll
-                        for (int iq = 0; iq < 4; iq++) he[3 * iq + ic] = hg_sum(W2, iq) * y;
-                    }
-                }
-            }
-        } else {
-#pragma unroll
-            for (int a = 0; a < L::NDIR; a++)
-#pragma unroll
-                for (int t = 0; t < 8; t++) cnb[a][t] = 0.f;
-        }
-#pragma unroll
-        for (int i = 0; i < 3; i++) { CELL(cs, i, tid) = ed[i]; CELL(cs, 3 + i, tid) = eo[i]; }
-#pragma unroll
-        for (int i = 0; i < 12; i++) CELL(cs, 6 + i, tid) = he[i];
-#pragma unroll
-        for (int a = 0; a < L::NDIR; a++)
-#pragma unroll
-            for (int t = 0; t < 8; t++) CELL(cs, 18 + 8 * a + t, tid) = cnb[a][t];
-    };
-
-    // ---------------------------------------------------------------- node phase
-    auto nodes = [&](int l, auto fast_tag) {
-        constexpr bool F = decltype(fast_tag)::value;
-        if (!outcol) return;
-        const long long q = g.idx(jn, kn, l);
-        // cells of diff_cn term t: (j-1|j, k-1|k, l-1|l)
-        int ci[8], cs[8];
-#pragma unroll
-        for (int t = 0; t < 8; t++) {
-            const int oj = (t & 1) ? 0 : -1, ok = (t >> 2) ? 0 : -1, ol = ((t >> 1) & 1) ? 0 : -1;
-            ci[t] = (tx + 1 + oj) + FJ * (ty + 1 + ok);
-            cs[t] = (l + ol) & 1;
-        }
-        float f[3];
-#pragma unroll
-        for (int ic = 0; ic < 3; ic++) {
-#pragma unroll
-            for (int iid = 0; iid < 3; iid++) {
-                const int id = (ic + iid) % 3;
-                const int comp = ic == id ? ic : 3 + (3 - ic - id);
-                float Fv[8], B[8];
-#pragma unroll
-                for (int t = 0; t < 8; t++) {
-                    Fv[t] = CELL(cs[t], comp, ci[t]);
-                    if (GEOM == GEOM_RECT || (GEOM == GEOM_TERRAIN && id == 2)) B[t] = FM ? A.brh.bcn[id][t] : A.br.bcn[id][t];
-                    else B[t] = CELL(cs[t], 18 + 8 * id + t, ci[t]);
-                }
-                float s = FM ? dot8(Fv, B) : stencil8(Fv, B, h);
-                if constexpr (!F) {
-                    const int c = id == 0 ? jn : id == 1 ? kn : l;
-                    if (c <= g.i1pml[id]) {
-                        const int p = c + g.nnoff[id];
-                        float* P = A.sl.p[id] + slab_idx(g, id, A.sl.tp[id], c - g.i1node[id], jn, kn, l, ic);
-                        s = A.pmlc[g.npml + p - 1] * s + A.pmlc[p - 1] * *P;
-                        *P = *P + dt * s;
-                    }
-                    if (c >= g.i2pml[id]) {
-                        const int p = g.nn[id] - c - g.nnoff[id] + 1;
-                        float* P = A.sl.p[3 + id] + slab_idx(g, id, A.sl.tp[3 + id], g.i2node[id] - c, jn, kn, l, ic);
-                        s = A.pmlc[g.npml + p - 1] * s + A.pmlc[p - 1] * *P;
-                        *P = *P + dt * s;
-                    }
-                }
-                f[ic] = iid == 0 ? s : f[ic] + s;
-            }
-        }
-        if (A.hourglass) {
-            bool ne = true;
-            if constexpr (!F) {
-                const int cn_[3] = {jn, kn, l};
-#pragma unroll
-                for (int d = 0; d < 3; d++) ne = ne && cn_[d] >= g.i1pml[d] + 1 && cn_[d] <= g.i2pml[d] - 1;
-            }
-            if (ne) {
-                int hi[8], hs[8];
-#pragma unroll
-                for (int t = 0; t < 8; t++) {
-                    const int o = hg_corner(t);
-                    hi[t] = (tx + 1 - (o & 1)) + FJ * (ty + 1 - ((o >> 1) & 1));
-                    hs[t] = (l - (o >> 2)) & 1;
-                }
-#pragma unroll
-                for (int iq = 0; iq < 4; iq++)
-#pragma unroll
-                    for (int ic = 0; ic < 3; ic++) {
-                        float H[8];
-#pragma unroll
-                        for (int t = 0; t < 8; t++) H[t] = CELL(hs[t], 6 + 3 * iq + ic, hi[t]);
-                        f[ic] = f[ic] - hg_sum(H, iq);
-                    }
-            } else if constexpr (!F) {
-                if (A.hgvisc) {
-                    // viscous-only hourglass in the PML (acceleration.f90:164-199):
-                    // every cell of a PML node is a PML cell; pure PML cells
-                    // hold their viscous values in the hourglass slots, cells
-                    // that are also elastic-hourglass cells (the layer next to
-                    // the elastic region) are evaluated here from v
-                    int hi[8], hs[8], kind[8];
-                    float yc[8];
-#pragma unroll
-                    for (int t = 0; t < 8; t++) {
-                        const int o = hg_corner(t);
-                        hi[t] = (tx + 1 - (o & 1)) + FJ * (ty + 1 - ((o >> 1) & 1));
-                        hs[t] = (l - (o >> 2)) & 1;
-                        const int Jc = jn - (o & 1), Kc = kn - ((o >> 1) & 1), Lc = l - (o >> 2);
-                        const bool real = Jc >= g.i1cell[0] && Jc <= g.i2cell[0] && Kc >= g.i1cell[1] &&
-                                          Kc <= g.i2cell[1] && Lc >= g.i1cell[2] && Lc <= g.i2cell[2];
-                        const bool slab = Jc <= g.i1pml[0] || Jc >= g.i2pml[0] - 1 || Kc <= g.i1pml[1] ||
-                                          Kc >= g.i2pml[1] - 1 || Lc <= g.i1pml[2] || Lc >= g.i2pml[2] - 1;
-                        const bool inEc = Jc >= g.i1pml[0] && Jc <= g.i2pml[0] - 1 && Kc >= g.i1pml[1] &&
-                                          Kc <= g.i2pml[1] - 1 && Lc >= g.i1pml[2] && Lc <= g.i2pml[2] - 1;
-                        kind[t] = !(real && slab) ? 0 : inEc ? 2 : 1;
-                        yc[t] = kind[t] == 2 ? A.dh2 * A.yy[g.idx(Jc, Kc, Lc)] : 0.f;
-                    }
-#pragma unroll 1
-                    for (int ic = 0; ic < 3; ic++) {
-                        float Hq[4][8];
-#pragma unroll
-                        for (int t = 0; t < 8; t++) {
-                            if (kind[t] == 1) {
-#pragma unroll
-                                for (int iq = 0; iq < 4; iq++) Hq[iq][t] = CELL(hs[t], 6 + 3 * iq + ic, hi[t]);
-                            } else if (kind[t] == 2) {
-                                const int o = hg_corner(t);
-                                float Vc[8];
-#pragma unroll
-                                for (int m = 0; m < 8; m++) {
-                                    const int n = hg_corner(m);
-                                    const int dj = (n & 1) - (o & 1), dk = ((n >> 1) & 1) - ((o >> 1) & 1),
-                                              dl = (n >> 2) - (o >> 2);
-                                    Vc[m] = A.vin[ic][g.idx(jn + dj, kn + dk, l + dl)];
-                                }
-#pragma unroll
-                                for (int iq = 0; iq < 4; iq++) Hq[iq][t] = yc[t] * hg_sum(Vc, iq);
-                            } else {
-#pragma unroll
-                                for (int iq = 0; iq < 4; iq++) Hq[iq][t] = 0.f;
-                            }
-                        }
-                        float fi = f[0];
-                        if (ic == 1) fi = f[1];
-                        if (ic == 2) fi = f[2];
-#pragma unroll
-                        for (int iq = 0; iq < 4; iq++) fi = fi - hg_sum(Hq[iq], iq);
-                        if (ic == 0) f[0] = fi;
-                        if (ic == 1) f[1] = fi;
-                        if (ic == 2) f[2] = fi;
-                    }
-                }
-            }
-        }
-        if constexpr (!F) {
-            const Inject* E = nfrc >= 0 ? lfrc : A.force.e;
-            const int n = nfrc >= 0 ? nfrc : A.force.n;
-            for (int e = 0; e < n; e++)
-                if (E[e].idx == q) {
-                    const int c = E[e].comp;
-                    const float inc = E[e].inc;
-                    if (c == 0) f[0] = f[0] + inc;
-                    else if (c == 1) f[1] = f[1] + inc;
-                    else f[2] = f[2] + inc;
-                }
-        }
-        finish_node<FM>(A, q, jn, kn, l, f, cur[4], uv, dt, st_a, st_v, st_u);
-    };
-
-    // ---------------------------------------------------------------- stream
-    // ring: planes L0-1, L0, L0+1; staged: L0+2 in flight
-#pragma unroll 1
-    for (int p = -1; p <= 1; p++) {
-        fetch(L0 + p);
-        cp_async_wait_all();
-        __syncthreads();
-        store((L0 + p + 3) % 3);
-        __syncthreads();
-    }
-    fetch(L0 + 2);
-    stat_load(L0 - 1, cur);
-    uv_load(L0, uv);
-    cells(L0 - 1, std::false_type{});
-    stat_load(L0, cur);
-#pragma unroll 1
-    for (int l = L0; l <= L1; l++) {
-        cells(l, std::false_type{});
-        float nxt[5], nuv[6];
-        stat_load(l + 1, nxt);
-        cp_async_wait_all();
-        __syncthreads();  // cell plane l complete, staged plane l+2 landed
-        store((l + 2) % 3);
-        nodes(l, std::false_type{});
-        uv_load(l + 1, nuv);
-        __syncthreads();  // ring slot l+2 complete, staging and cell slot l-1 free
-        fetch(l + 3);
-#pragma unroll
-        for (int i = 0; i < 5; i++) cur[i] = nxt[i];
-#pragma unroll
-        for (int i = 0; i < 6; i++) uv[i] = nuv[i];
-    }
-    cp_async_wait_all();
-    if (A.stats) {
-        bmax(A.red + 0, st_a);
-        bmax(A.red + 1, st_v);
-        bmax(A.red + 2, st_u);
-        bmax(A.red + 3, st_w);
-    }
-#undef RAW
-#undef NODE
-#undef CELL
-}
 
 // Zero one cell of the fast-arithmetic cell plane (layout of Lay: NGCF
 // groups of ncl float4) in the pattern the cell phase writes it: group 1
@@ -772,7 +218,7 @@ __device__ __forceinline__ void zero_cell_fr(float4* sC, int tid, int ncl) {
 // multiply-adds, brackets scaled by h once per cell, divergence brackets
 // taken as the negated gradient brackets; equal to the reference-order
 // kernel in exact arithmetic, not bit for bit.
-template <int GEOM, bool FASTK, bool FM>
+template <int GEOM, bool FM>
 __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(StepArgs A) {
     using L = Lay<GEOM>;
     constexpr int NGN = L::NGN, NGC = L::NGC, NDIR = L::NDIR;
@@ -806,18 +252,23 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
         tyb = A.y1d[K];
     }
 
-    // point injections that fall inside this block (cells / nodes it computes)
+    // point sources of the step in this block's box (cells j0-1.., nodes
+    // j0..); a block outside the box around all of them does not look, and
+    // only cells inside it do
     __shared__ Inject lpot[kLocalInject], lmom[kLocalInject], lfrc[kLocalInject];
     __shared__ int lcnt[3];
-    // A fast-kernel block whose (j, k) box holds a point source of this step
-    // leaves that column to the general kernel (the host lists it there).
-    const int gl1 = FASTK ? 0 : L0 - 1, gl2 = FASTK ? g.nm[2] + 1 : L1;
-    gather_inject(A.pot, lpot, &lcnt[0], g, j0 - 1, j0 + FOJ - 1, k0 - 1, k0 + FOK - 1, gl1, gl2);
-    gather_inject(A.mom, lmom, &lcnt[1], g, j0 - 1, j0 + FOJ - 1, k0 - 1, k0 + FOK - 1, gl1, gl2);
-    gather_inject(A.force, lfrc, &lcnt[2], g, j0, j0 + FOJ - 1, k0, k0 + FOK - 1, FASTK ? gl1 : L0, gl2);
-    __syncthreads();
-    const int npot = lcnt[0], nmom = lcnt[1], nfrc = lcnt[2];
-    if (FASTK && (npot != 0 || nmom != 0 || nfrc != 0)) return;
+    int npot = 0, nmom = 0, nfrc = 0;
+    if (A.ibox[0] <= j0 + FOJ - 1 && A.ibox[3] >= j0 - 1 && A.ibox[1] <= k0 + FOK - 1 && A.ibox[4] >= k0 - 1 &&
+        A.ibox[2] <= L1 && A.ibox[5] >= L0 - 1) {
+        gather_inject(A.pot, lpot, &lcnt[0], g, j0 - 1, j0 + FOJ - 1, k0 - 1, k0 + FOK - 1, L0 - 1, L1);
+        gather_inject(A.mom, lmom, &lcnt[1], g, j0 - 1, j0 + FOJ - 1, k0 - 1, k0 + FOK - 1, L0 - 1, L1);
+        gather_inject(A.force, lfrc, &lcnt[2], g, j0, j0 + FOJ - 1, k0, k0 + FOK - 1, L0, L1);
+        __syncthreads();
+        npot = lcnt[0];
+        nmom = lcnt[1];
+        nfrc = lcnt[2];
+    }
+    const bool scol = (npot != 0 || nmom != 0) && J >= A.ibox[0] && J <= A.ibox[3] && K >= A.ibox[1] && K <= A.ibox[4];
 
     // ---------------------------------------------------------------- loads
     // stage node plane l (u, v, gam, coordinates) into sR asynchronously
@@ -1170,7 +621,15 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
                     else eo[3 - ic - id] = eo[3 - ic - id] + 0.5f * s;
                 }
             }
-            apply_inject(lpot, npot, A.pot, q, ed, eo);
+        }
+        const bool src = scol && l >= A.ibox[2] && l <= A.ibox[5];
+        if (src && npot != 0) {
+            // strain (fast arithmetic carries the off-diagonal terms twice)
+            float pd[3] = {0.f, 0.f, 0.f}, po[3] = {0.f, 0.f, 0.f};
+            apply_inject(lpot, npot, A.pot, q, FM ? pd : ed, FM ? po : eo);
+            if (FM)
+#pragma unroll
+                for (int i = 0; i < 3; i++) { ed[i] = ed[i] + pd[i]; eo[i] = fmaf(2.0f, po[i], eo[i]); }
         }
         if constexpr (FM) {
             // (2 mu e + lam tr e) / V; the off-diagonal sums carry the 1/2
@@ -1178,6 +637,12 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
             const float s1r = (cur[0] * r) * (ed[0] + ed[1] + ed[2]);
 #pragma unroll
             for (int i = 0; i < 3; i++) { ed[i] = fmaf(m2r, ed[i], s1r); eo[i] = mur * eo[i]; }
+            if (src && nmom != 0) {
+                float pd[3] = {0.f, 0.f, 0.f}, po[3] = {0.f, 0.f, 0.f};
+                apply_inject(lmom, nmom, A.mom, q, pd, po);
+#pragma unroll
+                for (int i = 0; i < 3; i++) { ed[i] = fmaf(pd[i], r, ed[i]); eo[i] = fmaf(po[i], r, eo[i]); }
+            }
         } else {
             {
                 const float lm = cur[0], m2 = 2.0f * cur[1];
@@ -1185,7 +650,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
 #pragma unroll
                 for (int i = 0; i < 3; i++) { ed[i] = m2 * ed[i] + s1v; eo[i] = m2 * eo[i]; }
             }
-            if constexpr (!F) apply_inject(lmom, nmom, A.mom, q, ed, eo);
+            if (src) apply_inject(lmom, nmom, A.mom, q, ed, eo);
             {
                 const float r = cur[2];
 #pragma unroll
@@ -1288,6 +753,21 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
         } else {
             WRITE_CELL(cs, ed, eo, he, cnb);
         }
+    };
+
+    // force sources at node q
+    auto add_force = [&](long long q, float (&f)[3]) {
+        if (nfrc == 0) return;
+        const Inject* E = nfrc >= 0 ? lfrc : A.force.e;
+        const int n = nfrc >= 0 ? nfrc : A.force.n;
+        for (int e = 0; e < n; e++)
+            if (E[e].idx == q) {
+                const int c = E[e].comp;
+                const float inc = E[e].inc;
+                if (c == 0) f[0] = f[0] + inc;
+                else if (c == 1) f[1] = f[1] + inc;
+                else f[2] = f[2] + inc;
+            }
     };
 
     // ---------------------------------------------------------------- node phase
@@ -1530,18 +1010,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
                 }
             }
         }
-        if constexpr (!F) {
-            const Inject* E = nfrc >= 0 ? lfrc : A.force.e;
-            const int n = nfrc >= 0 ? nfrc : A.force.n;
-            for (int e = 0; e < n; e++)
-                if (E[e].idx == q) {
-                    const int c = E[e].comp;
-                    const float inc = E[e].inc;
-                    if (c == 0) f[0] = f[0] + inc;
-                    else if (c == 1) f[1] = f[1] + inc;
-                    else f[2] = f[2] + inc;
-                }
-        }
+        add_force(q, f);
         finish_node<FM>(A, q, jn, kn, l, f, cur[4], uv, dt, st_a, st_v, st_u);
     };
 
@@ -1573,12 +1042,13 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
 #pragma unroll
         for (int i = 0; i < 3; i++) fc[i] = fl[i];
         if (!finish) return;
+        add_force(g.idx(jn, kn, l), fu);
         finish_node<FM>(A, g.idx(jn, kn, l), jn, kn, l, fu, cur[4], uv, dt, st_a, st_v, st_u);
     };
 
     // ---------------------------------------------------------------- stream
     // ring: planes L0-1, L0, L0+1; staged: L0+2 in flight
-    constexpr std::integral_constant<bool, FASTK> path{};
+    constexpr std::true_type path{};
 #pragma unroll 1
     for (int p = -1; p <= 1; p++) {
         fetch(L0 + p);
@@ -1590,30 +1060,27 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
     fetch(L0 + 2);
     stat_load(L0 - 1, cur);
     uv_load(L0, uv);
-    cells(L0 - 1, path);
-    if constexpr (FM) {
-        __syncthreads();  // cell plane L0-1 complete: its terms for node L0
-        nodes_fm(L0 - 1, false);
-        __syncthreads();  // one cell slot: read before cells(L0) overwrites it
-    }
-    stat_load(L0, cur);
+    // (one call of cells and of each node phase, so that all are inlined)
 #pragma unroll 1
-    for (int l = L0; l <= L1; l++) {
+    for (int l = L0 - 1; l <= L1; l++) {
+        const bool first = l < L0;  // the cell plane below the first node plane
         cells(l, path);
         float nxt[5], nuv[6];
         stat_load(l + 1, nxt);
-        cp_async_wait_all();
+        if (!first) cp_async_wait_all();
         __syncthreads();  // cell plane l complete, staged plane l+2 landed
-        store((l + 2) % 3);
-        if constexpr (FM) nodes_fm(l, true);
-        else nodes(l, path);
-        uv_load(l + 1, nuv);
+        if (!first) store((l + 2) % 3);
+        if constexpr (FM) nodes_fm(l, !first);
+        else if (!first) nodes(l, path);
+        if (!first) uv_load(l + 1, nuv);
         __syncthreads();  // ring slot l+2 complete, staging and cell slot l-1 free
-        fetch(l + 3);
+        if (!first) {
+            fetch(l + 3);
+#pragma unroll
+            for (int i = 0; i < 6; i++) uv[i] = nuv[i];
+        }
 #pragma unroll
         for (int i = 0; i < 5; i++) cur[i] = nxt[i];
-#pragma unroll
-        for (int i = 0; i < 6; i++) uv[i] = nuv[i];
     }
     cp_async_wait_all();
     if (A.stats) {
@@ -1628,13 +1095,8 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
 }
 
 #include "modal.cuh"
+#include "shell.cuh"
 #include "slab.cuh"
-
-// A region of shell items made by one push_box call: boxes of 15 x 15
-// nodes from (j1, k1) and ipl planes from l1, l outermost, j innermost.
-struct BoxRegion {
-    int j1, k1, l1, j2, k2, l2, ipl, nbj, nbk, nbl, first;
-};
 
 // Work decomposition of a fused step, fixed by the mesh.  The interior
 // rectangle holds the node columns (j, k) whose adjacent cells all lie
@@ -1642,9 +1104,8 @@ struct BoxRegion {
 // 31 x 7 node tiles from (jf, kf) (the last tile of a row may be partial)
 // and runs the interior kernel over the node planes lf0..lf1 whose cells are
 // interior (or the halo plane of a free surface).  Everything else -- the
-// PML faces at full depth, the PML planes of the interior rectangle, and in
-// each step the interior tiles holding a point source -- is covered by
-// masked 15 x 15 node boxes for the shell kernel.  Boxes and tiles partition
+// PML faces at full depth and the PML planes of the interior rectangle -- is
+// covered by masked 15 x 15 node boxes for the shell kernel.  Boxes and tiles partition
 // the nodes, so every node, and every PML memory, is updated once.
 struct FusedPlan {
     int arith = 0;                              // the arithmetic it was made for
@@ -1652,20 +1113,15 @@ struct FusedPlan {
     int nbx = 0, nby = 0;                       // interior tiles
     int lf0 = 0, lf1 = -1;                      // interior node planes (inclusive)
     int segl = 0, nseg = 1;                     // interior planes per block, blocks per column
-    int ipl = 16;                               // planes per item of a point-source tile
-    std::vector<int> base;                      // shell items without point sources (6 ints each)
-    std::vector<int> bmask;                     // per base item: k_slab class (0..3: MASK 1, 2, 4, 7)
-    std::vector<BoxRegion> regions;             // how the base items were laid out
-    std::vector<int> cur;                       // items of the last upload
+    // node boxes of the PML shell, six ints each (j0, k0, last j, last k,
+    // first and last plane), by class of damped axes (MASK 1, 2, 4, 7)
+    int nbox[4] = {0, 0, 0, 0};
     int* d_items = nullptr;
-    int* h_items = nullptr;                     // pinned staging
-    int cap = 0;                                // items
-    cudaEvent_t done = nullptr;
     // the PML-shell kernel runs on a second stream, concurrently with the
     // interior kernel (they write disjoint nodes and read the same inputs)
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
-    // each k_slab class on its own stream, forked from and joined back into
+    // each class of boxes on its own stream, forked from and joined back into
     // the stream of the shell launches, so that the classes' tails overlap
     cudaStream_t cst[4] = {};
     cudaEvent_t cfork = nullptr, cdone[4] = {};
@@ -1674,7 +1130,6 @@ struct FusedPlan {
 void fused_free(Solver& s) {
     FusedPlan* P = s.fplan;
     if (!P) return;
-    if (P->done) cudaEventDestroy(P->done);
     if (P->fork) cudaEventDestroy(P->fork);
     if (P->join) cudaEventDestroy(P->join);
     if (P->side) cudaStreamDestroy(P->side);
@@ -1684,7 +1139,6 @@ void fused_free(Solver& s) {
         if (P->cst[c]) cudaStreamDestroy(P->cst[c]);
     }
     dev_free(s, P->d_items);
-    pinned_put(P->h_items);
     delete P;
     s.fplan = nullptr;
 }
@@ -1699,17 +1153,9 @@ static constexpr int kItemPlanes = 96;
 static constexpr int kMinPlanes = 8;
 static constexpr int kFewPlanes = 4;
 static constexpr int kWaveBlocks = 4;
-// planes per item of an interior tile holding a point source (k_shell): a
-// few tile columns only, so short items spread them over the SMs
-static constexpr int kSourcePlanes = 16;
 
 // shell items covering node box [j1, j2] x [k1, k2] x [l1, l2]
-static void push_box(std::vector<int>& v, int ipl, int j1, int j2, int k1, int k2, int l1, int l2,
-                     std::vector<BoxRegion>* reg = nullptr) {
-    if (j1 > j2 || k1 > k2 || l1 > l2) return;
-    if (reg)
-        reg->push_back({j1, k1, l1, j2, k2, l2, ipl, (j2 - j1) / (SJ - 1) + 1, (k2 - k1) / (SK - 1) + 1,
-                        (l2 - l1) / ipl + 1, (int)v.size() / 6});
+static void push_box(std::vector<int>& v, int ipl, int j1, int j2, int k1, int k2, int l1, int l2) {
     for (int a = l1; a <= l2; a += ipl)
         for (int k = k1; k <= k2; k += SK - 1)
             for (int j = j1; j <= j2; j += SJ - 1) {
@@ -1757,7 +1203,7 @@ static FusedPlan& fused_plan(Solver& s) {
     SORD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.device));
     const int want = kWaveBlocks * sms;
     // regions of the shell, cut where the PML of another axis begins so that
-    // each is damped along as few axes as possible (its k_slab class)
+    // each is damped along as few axes as possible (its class)
     struct RegionBox {
         int lo[3], hi[3];
     };
@@ -1782,7 +1228,7 @@ static FusedPlan& fused_plan(Solver& s) {
         add(P->jf, P->jend, P->kf, P->kend, L1, P->lf0 - 1);
         add(P->jf, P->jend, P->kf, P->kend, P->lf1 + 1, L2);
     }
-    // k_slab class of a node box: axis d needs the PML terms when a real cell
+    // class of a node box: axis d needs the PML terms when a real cell
     // the box computes (node range a..b -> cells a-1..b) or one of its real
     // nodes lies in a PML slab of d; one axis -> its own class, more -> all
     auto klass = [&](const int* lo, const int* hi) {
@@ -1816,15 +1262,20 @@ static FusedPlan& fused_plan(Solver& s) {
         while (ipl > few && count(ipl) < sms) ipl = std::max(few, ipl * 2 / 3);
         iplc[c] = ipl;
     }
-    P->regions.clear();
+    // boxes by their own class (a range of planes may miss the PML of z)
+    std::vector<int> boxes, byclass[4];
     for (size_t i = 0; i < rb.size(); i++)
-        push_box(P->base, iplc[rcls[i]], rb[i].lo[0], rb[i].hi[0], rb[i].lo[1], rb[i].hi[1], rb[i].lo[2], rb[i].hi[2],
-                 &P->regions);
-    P->ipl = kSourcePlanes;
-    for (size_t i = 0; i < P->base.size(); i += 6) {
-        const int* b = &P->base[i];
+        push_box(boxes, iplc[rcls[i]], rb[i].lo[0], rb[i].hi[0], rb[i].lo[1], rb[i].hi[1], rb[i].lo[2], rb[i].hi[2]);
+    for (size_t i = 0; i < boxes.size(); i += 6) {
+        const int* b = &boxes[i];
         const int lo[3] = {b[0], b[1], b[4]}, hi[3] = {b[2], b[3], b[5]};
-        P->bmask.push_back(klass(lo, hi));
+        std::vector<int>& v = byclass[klass(lo, hi)];
+        v.insert(v.end(), b, b + 6);
+    }
+    std::vector<int> items;
+    for (int c = 0; c < 4; c++) {
+        P->nbox[c] = (int)byclass[c].size() / 6;
+        items.insert(items.end(), byclass[c].begin(), byclass[c].end());
     }
     if (!inner) {
         P->jend = P->jf - 1;
@@ -1833,9 +1284,10 @@ static FusedPlan& fused_plan(Solver& s) {
         P->nby = (int)div_up(P->kend - P->kf + 1, FOK);
         const int planes = P->lf1 - P->lf0 + 1, cols = P->nbx * P->nby;
         // the split that takes the fewest plane times: rounds of two blocks
-        // per SM, each block its planes and a prologue of about two (aiming
-        // at four blocks per SM instead left a third round of 56 blocks on
-        // 203 x 149 x 97 nodes)
+        // per SM, each block its planes and a prologue of about two.  (An
+        // even spread with half a last round, as if blocks did not come in
+        // rounds, splits further: 5 % slower on 256 x 256 x 128 nodes in
+        // reference order, where the shell's blocks fill the gaps anyway.)
         double best = 0;
         for (int n = 1; n <= std::max(1, planes / few); n++) {
             const int len = (planes + n - 1) / n;
@@ -1848,10 +1300,11 @@ static FusedPlan& fused_plan(Solver& s) {
         }
         P->nseg = (planes + P->segl - 1) / P->segl;
     }
-    P->cap = (int)P->base.size() / 6 + 16384;
-    SORD_CUDA(dev_malloc(s, (void**)&P->d_items, sizeof(int) * 6 * P->cap));
-    P->h_items = (int*)pinned_get(sizeof(int) * 6 * P->cap);
-    SORD_CUDA(cudaEventCreateWithFlags(&P->done, cudaEventDisableTiming));
+    SORD_CUDA(dev_malloc(s, (void**)&P->d_items, sizeof(int) * std::max<size_t>(items.size(), 6)));
+    if (!items.empty()) {
+        SORD_CUDA(cudaMemcpyAsync(P->d_items, items.data(), sizeof(int) * items.size(), cudaMemcpyHostToDevice, s.stream));
+        SORD_CUDA(cudaStreamSynchronize(s.stream));
+    }
     SORD_CUDA(cudaEventCreateWithFlags(&P->fork, cudaEventDisableTiming));
     SORD_CUDA(cudaEventCreateWithFlags(&P->join, cudaEventDisableTiming));
     SORD_CUDA(cudaStreamCreateWithFlags(&P->side, cudaStreamNonBlocking));
@@ -1863,25 +1316,6 @@ static FusedPlan& fused_plan(Solver& s) {
     return *P;
 }
 
-// Interior tiles whose (j, k) box holds a point source of this step; the
-// boxes are those the interior kernel tests (cells j0-1..j0+30 for potency /
-// moment entries, nodes j0..j0+30 for forces), so both sides agree.
-static void source_tiles(const Solver& s, const FusedPlan& P, const std::vector<Inject>& e, bool cell,
-                         std::vector<std::pair<int, int>>& out) {
-    const Geom& g = s.g;
-    for (const Inject& x : e) {
-        const int j = (int)(x.idx % g.sy) + 1, k = (int)((x.idx / g.sy) % g.nm[1]) + 1;
-        for (int bx = 0; bx < P.nbx; bx++) {
-            const int j0 = P.jf + bx * FOJ;
-            if (!(cell ? (j >= j0 - 1 && j <= j0 + FOJ - 1) : (j >= j0 && j <= j0 + FOJ - 1))) continue;
-            for (int by = 0; by < P.nby; by++) {
-                const int k0 = P.kf + by * FOK;
-                if (cell ? (k >= k0 - 1 && k <= k0 + FOK - 1) : (k >= k0 && k <= k0 + FOK - 1)) out.push_back({bx, by});
-            }
-        }
-    }
-}
-
 template <int GEOM, int MASK>
 static void launch_modal(Solver& s, const StepArgs& A, dim3 grid, cudaStream_t st) {
     using L = LayM<MASK>;
@@ -1891,29 +1325,6 @@ static void launch_modal(Solver& s, const StepArgs& A, dim3 grid, cudaStream_t s
     } else {
         smem_limit((const void*)k_modal<GEOM, MASK, false>, (int)L::bytes);
         k_modal<GEOM, MASK, false><<<grid, dim3(L::TJ, L::TK), L::bytes, st>>>(A);
-    }
-    s.launches++;
-    SORD_CUDA(cudaGetLastError());
-}
-
-template <int GEOM, bool FASTK>
-static void launch_mode(Solver& s, const StepArgs& A, dim3 grid, cudaStream_t st) {
-    // fast arithmetic: k_modal, on general meshes k_interior and k_shell
-    constexpr bool FM = GEOM == GEOM_GENERAL;
-    if constexpr (FASTK) {
-        if (s.arith && !FM) {
-            launch_modal<GEOM, 0>(s, A, grid, st);
-            return;
-        }
-        const size_t bytes = FM && s.arith ? Lay<GEOM>::bytes_fm : Lay<GEOM>::bytes;
-        auto kern = FM && s.arith ? k_interior<GEOM, true, FM> : k_interior<GEOM, true, false>;
-        smem_limit((const void*)kern, (int)bytes);
-        kern<<<grid, dim3(FJ, FK), bytes, st>>>(A);
-    } else {
-        const size_t bytes = LayS<GEOM, (SJ + 1) * (SK + 1), SJ * SK>::bytes;
-        auto kern = FM && s.arith ? k_shell<GEOM, FM> : k_shell<GEOM, false>;
-        smem_limit((const void*)kern, (int)bytes);
-        kern<<<grid, dim3(SJ, SK), bytes, st>>>(A);
     }
     s.launches++;
     SORD_CUDA(cudaGetLastError());
@@ -1943,40 +1354,51 @@ static int step_class(const Solver& s) {
     return GEOM_RECT;
 }
 
-template <int GEOM, int MASK>
-static void launch_slab_m(Solver& s, const StepArgs& A, unsigned n, cudaStream_t st) {
-    if constexpr (GEOM != GEOM_GENERAL) {
-        launch_modal<GEOM, MASK>(s, A, dim3(n, 1, 1), st);
-    } else {
-        const size_t bytes = LaySl::bytes;
-        smem_limit((const void*)k_slab<MASK>, (int)bytes);
-        k_slab<MASK><<<dim3(n, 1, 1), dim3(SJ, SK), bytes, st>>>(A);
-        s.launches++;
-        SORD_CUDA(cudaGetLastError());
+// Interior tiles.
+template <int GEOM>
+static void launch_interior(Solver& s, const StepArgs& A, dim3 grid, cudaStream_t st) {
+    constexpr bool FM = GEOM == GEOM_GENERAL;  // fast arithmetic of the other meshes: k_modal
+    if constexpr (!FM) {
+        if (s.arith) {
+            launch_modal<GEOM, 0>(s, A, grid, st);
+            return;
+        }
     }
+    const size_t bytes = FM && s.arith ? Lay<GEOM>::bytes_fm : Lay<GEOM>::bytes;
+    auto kern = FM && s.arith ? k_interior<GEOM, FM> : k_interior<GEOM, false>;
+    smem_limit((const void*)kern, (int)bytes);
+    kern<<<grid, dim3(FJ, FK), bytes, st>>>(A);
+    s.launches++;
+    SORD_CUDA(cudaGetLastError());
+}
+
+// Boxes of the PML shell of one class.
+template <int GEOM, int MASK>
+static void launch_boxes(Solver& s, const StepArgs& A, unsigned n, cudaStream_t st) {
+    if (s.arith) {
+        if constexpr (GEOM != GEOM_GENERAL) {
+            launch_modal<GEOM, MASK>(s, A, dim3(n, 1, 1), st);
+            return;
+        } else {
+            const size_t bytes = LaySl::bytes;
+            smem_limit((const void*)k_slab<MASK>, (int)bytes);
+            k_slab<MASK><<<dim3(n, 1, 1), dim3(SJ, SK), bytes, st>>>(A);
+        }
+    } else {
+        const size_t bytes = LaySh<GEOM>::bytes;
+        smem_limit((const void*)k_shell<GEOM, MASK>, (int)bytes);
+        k_shell<GEOM, MASK><<<dim3(n, 1, 1), dim3(SJ, SK), bytes, st>>>(A);
+    }
+    s.launches++;
+    SORD_CUDA(cudaGetLastError());
 }
 
 template <int GEOM>
-static void launch_slab_g(Solver& s, const StepArgs& A, int cls, unsigned n, cudaStream_t st) {
-    if (cls == 0) launch_slab_m<GEOM, 1>(s, A, n, st);
-    else if (cls == 1) launch_slab_m<GEOM, 2>(s, A, n, st);
-    else if (cls == 2) launch_slab_m<GEOM, 4>(s, A, n, st);
-    else launch_slab_m<GEOM, 7>(s, A, n, st);
-}
-
-static void launch_slab(Solver& s, const StepArgs& A, int cls, unsigned n, cudaStream_t st) {
-    const int geom = step_class(s);
-    if (geom == GEOM_RECT) launch_slab_g<GEOM_RECT>(s, A, cls, n, st);
-    else if (geom == GEOM_TERRAIN) launch_slab_g<GEOM_TERRAIN>(s, A, cls, n, st);
-    else launch_slab_g<GEOM_GENERAL>(s, A, cls, n, st);
-}
-
-template <bool FASTK>
-static void launch_geom(Solver& s, const StepArgs& A, dim3 grid, cudaStream_t st) {
-    const int geom = FASTK ? step_class(s) : s.geom;
-    if (geom == GEOM_RECT) launch_mode<GEOM_RECT, FASTK>(s, A, grid, st);
-    else if (geom == GEOM_TERRAIN) launch_mode<GEOM_TERRAIN, FASTK>(s, A, grid, st);
-    else launch_mode<GEOM_GENERAL, FASTK>(s, A, grid, st);
+static void launch_class(Solver& s, const StepArgs& A, int cls, unsigned n, cudaStream_t st) {
+    if (cls == 0) launch_boxes<GEOM, 1>(s, A, n, st);
+    else if (cls == 1) launch_boxes<GEOM, 2>(s, A, n, st);
+    else if (cls == 2) launch_boxes<GEOM, 4>(s, A, n, st);
+    else launch_boxes<GEOM, 7>(s, A, n, st);
 }
 
 // The statics of k_modal, laid out anew where they are not valid.
@@ -2057,115 +1479,46 @@ void launch_fused(Solver& s, const InjectList& pot, const InjectList& mom, const
         }
     for (int d = 0; d < 6; d++) A.ibox[d] = ib[d];
 
-    // shell items of this step: the fixed list, plus the interior planes of
-    // the interior tiles holding a point source
-    // (k_modal applies point sources itself)
-    const bool modal = s.arith && step_class(s) != GEOM_GENERAL;
-    A.sta = modal ? modal_statics(s) : nullptr;
-    std::vector<std::pair<int, int>> src;
-    if (P.nbx > 0 && !modal) {
-        source_tiles(s, P, hpot, true, src);
-        source_tiles(s, P, hmom, true, src);
-        source_tiles(s, P, hforce, false, src);
-        std::sort(src.begin(), src.end());
-        src.erase(std::unique(src.begin(), src.end()), src.end());
-    }
-    // In fast arithmetic the boxes without a point source go to k_slab (all of
-    // them to k_modal, which applies point sources itself), by
-    // class; k_shell takes the rest (the boxes k_shell tests: cells
-    // j0-1..j0+14 for potency / moment entries, nodes j0..j0+14 for forces).
-    // Upload order: k_shell items, then the k_slab classes.
-    const int nbase = (int)P.base.size() / 6;
-    std::vector<char> hit(nbase, s.arith ? 0 : 1);
-    if (s.arith && !modal) {
-        // an entry at (j, k, l) reaches box (j0, k0, L0..L1) when
-        // j0 - o <= j <= j0 + 14 (o = 1 for cells), likewise k, and
-        // L0 - o <= l <= L1: at most two boxes per axis in each region
-        auto mark = [&](const std::vector<Inject>& e, bool cell) {
-            const int o = cell ? 1 : 0;
-            auto span = [](int x, int x1, int step, int n, int lo, int hi, int& a, int& b) {
-                // boxes i (origin x1 + step i) with origin + lo <= x <= origin + hi
-                a = std::max(0, (int)std::ceil((double)(x - hi - x1) / step));
-                b = std::min(n - 1, (int)std::floor((double)(x - lo - x1) / step));
-            };
-            for (const Inject& x : e) {
-                const int j = (int)(x.idx % s.g.sy) + 1, k = (int)((x.idx / s.g.sy) % s.g.nm[1]) + 1;
-                const int l = (int)(x.idx / s.g.sz) + 1;
-                for (const BoxRegion& r : P.regions) {
-                    int ja, jb, ka, kb, la, lb;
-                    span(j, r.j1, SJ - 1, r.nbj, -o, SJ - 2, ja, jb);
-                    span(k, r.k1, SK - 1, r.nbk, -o, SK - 2, ka, kb);
-                    span(l, r.l1, r.ipl, r.nbl, -o, r.ipl - 1, la, lb);
-                    for (int bl = la; bl <= lb; bl++)
-                        for (int bk = ka; bk <= kb; bk++)
-                            for (int bj = ja; bj <= jb; bj++) {
-                                const int i = r.first + (bl * r.nbk + bk) * r.nbj + bj;
-                                if (l <= P.base[6 * i + 5]) hit[i] = 1;
-                            }
-                }
-            }
-        };
-        mark(hpot, true);
-        mark(hmom, true);
-        mark(hforce, false);
-    }
-    std::vector<int> items;
-    for (int i = 0; i < nbase; i++)
-        if (hit[i]) items.insert(items.end(), P.base.begin() + 6 * i, P.base.begin() + 6 * i + 6);
-    for (auto& c : src) {
-        const int j0 = P.jf + c.first * FOJ, k0 = P.kf + c.second * FOK;
-        push_box(items, P.ipl, j0, std::min(P.jend, j0 + FOJ - 1), k0, std::min(P.kend, k0 + FOK - 1), P.lf0, P.lf1);
-    }
-    const int nshell = (int)items.size() / 6;
-    int nslab[4] = {0, 0, 0, 0};
-    for (int m = 0; m < 4; m++)
-        for (int i = 0; i < nbase; i++)
-            if (!hit[i] && P.bmask[i] == m) {
-                items.insert(items.end(), P.base.begin() + 6 * i, P.base.begin() + 6 * i + 6);
-                nslab[m]++;
-            }
-    const int nitems = (int)items.size() / 6;
-    if (items != P.cur) {
-        if (nitems > P.cap) throw SordError(SORD_E_PARAM, "too many point-source tiles in one step");
-        SORD_CUDA(cudaEventSynchronize(P.done));
-        std::memcpy(P.h_items, items.data(), sizeof(int) * items.size());
-        SORD_CUDA(cudaMemcpyAsync(P.d_items, P.h_items, sizeof(int) * items.size(), cudaMemcpyHostToDevice, s.stream));
-        SORD_CUDA(cudaEventRecord(P.done, s.stream));
-        P.cur = items;
-    }
+    const int geom = step_class(s);
+    A.sta = s.arith && geom != GEOM_GENERAL ? modal_statics(s) : nullptr;
 
     cudaEvent_t e0 = nullptr;
     s.prof_begin(KC_FUSED, &e0);
     const bool inner = P.nbx > 0 && P.nby > 0;
     const dim3 igrid(P.nbx, P.nby, P.nseg);
-    // the shell launches: k_shell and beside it each class.  The classes are
-    // forked before k_shell, whose few source boxes would hold them up
-    // (160 x 144 x 120 perturbed mesh: 640 -> 562 us a step)
+    // the shell: each class on its own stream
     auto shell_launches = [&](cudaStream_t st) {
         SORD_CUDA(cudaEventRecord(P.cfork, st));
-        if (nshell > 0) launch_geom<false>(s, A, dim3((unsigned)nshell, 1, 1), st);
-        int off = nshell;
+        int off = 0;
         for (int m = 0; m < 4; m++) {
-            if (nslab[m] == 0) continue;
+            if (P.nbox[m] == 0) continue;
             StepArgs B = A;
             B.items = P.d_items + 6 * (size_t)off;
             SORD_CUDA(cudaStreamWaitEvent(P.cst[m], P.cfork, 0));
-            launch_slab(s, B, m, (unsigned)nslab[m], P.cst[m]);
+            if (geom == GEOM_RECT) launch_class<GEOM_RECT>(s, B, m, (unsigned)P.nbox[m], P.cst[m]);
+            else if (geom == GEOM_TERRAIN) launch_class<GEOM_TERRAIN>(s, B, m, (unsigned)P.nbox[m], P.cst[m]);
+            else launch_class<GEOM_GENERAL>(s, B, m, (unsigned)P.nbox[m], P.cst[m]);
             SORD_CUDA(cudaEventRecord(P.cdone[m], P.cst[m]));
             SORD_CUDA(cudaStreamWaitEvent(st, P.cdone[m], 0));
-            off += nslab[m];
+            off += P.nbox[m];
         }
     };
-    if (inner && nitems > 0) {
+    auto interior = [&]() {
+        if (geom == GEOM_RECT) launch_interior<GEOM_RECT>(s, A, igrid, s.stream);
+        else if (geom == GEOM_TERRAIN) launch_interior<GEOM_TERRAIN>(s, A, igrid, s.stream);
+        else launch_interior<GEOM_GENERAL>(s, A, igrid, s.stream);
+    };
+    const bool shell = P.nbox[0] + P.nbox[1] + P.nbox[2] + P.nbox[3] > 0;
+    if (inner && shell) {
         SORD_CUDA(cudaEventRecord(P.fork, s.stream));
         SORD_CUDA(cudaStreamWaitEvent(P.side, P.fork, 0));
         shell_launches(P.side);
-        launch_geom<true>(s, A, igrid, s.stream);
+        interior();
         SORD_CUDA(cudaEventRecord(P.join, P.side));
         SORD_CUDA(cudaStreamWaitEvent(s.stream, P.join, 0));
     } else if (inner) {
-        launch_geom<true>(s, A, igrid, s.stream);
-    } else if (nitems > 0) {
+        interior();
+    } else if (shell) {
         shell_launches(s.stream);
     }
     s.prof_end(KC_FUSED, e0);

@@ -42,54 +42,6 @@
 // (203 x 149 x 97 terrain, interior).
 #pragma once
 
-// A vector, operated on by component.
-struct M3 {
-    float x, y, z;
-};
-__device__ __forceinline__ M3 operator+(const M3& a, const M3& b) { return M3{a.x + b.x, a.y + b.y, a.z + b.z}; }
-__device__ __forceinline__ M3 operator-(const M3& a, const M3& b) { return M3{a.x - b.x, a.y - b.y, a.z - b.z}; }
-__device__ __forceinline__ M3 operator-(const M3& a) { return M3{-a.x, -a.y, -a.z}; }
-__device__ __forceinline__ M3 operator*(float a, const M3& b) { return M3{a * b.x, a * b.y, a * b.z}; }
-__device__ __forceinline__ M3 m_fma(float a, const M3& b, const M3& c) {
-    return M3{fmaf(a, b.x, c.x), fmaf(a, b.y, c.y), fmaf(a, b.z, c.z)};
-}
-
-// Sums of one mode pair: p keeps its sign across the cell, q changes it.
-// T completes the lower plane, acc starts the upper one.
-template <bool P, bool Q>
-__device__ __forceinline__ void m_two(const M3& p, const M3& q, M3& acc, M3& T) {
-    if (P && Q) {
-        T = acc + (p - q);
-        acc = p + q;
-    } else if (P) {
-        T = acc + p;
-        acc = p;
-    } else if (Q) {
-        T = acc - q;
-        acc = q;
-    }
-}
-// Corner values (0,0) (1,0) (0,1) (1,1) of plane sums T = (const, j, k, jk);
-// HAS bit m: T[m] is not zero.
-template <int HAS>
-__device__ __forceinline__ void m_corners(const M3 (&T)[4], M3 (&f)[4]) {
-    constexpr bool C = HAS & 1, Jm = HAS & 2, Km = HAS & 4, JK = HAS & 8;
-    M3 a0{}, a1{}, b0{}, b1{};
-    if (C && Km) { a0 = T[0] - T[2]; a1 = T[0] + T[2]; }
-    else if (C) { a0 = T[0]; a1 = T[0]; }
-    else if (Km) { a0 = -(T[2]); a1 = T[2]; }
-    if (Jm && JK) { b0 = T[1] - T[3]; b1 = T[1] + T[3]; }
-    else if (Jm) { b0 = T[1]; b1 = T[1]; }
-    else if (JK) { b0 = -(T[3]); b1 = T[3]; }
-    if ((C || Km) && (Jm || JK)) {
-        f[0] = a0 - b0; f[1] = a0 + b0; f[2] = a1 - b1; f[3] = a1 + b1;
-    } else if (C || Km) {
-        f[0] = a0; f[1] = a0; f[2] = a1; f[3] = a1;
-    } else {
-        f[0] = -(b0); f[1] = b0; f[2] = -(b1); f[3] = b1;
-    }
-}
-
 // Tile of a block: TJ x TK cells, one per thread, (TJ - 1) x (TK - 1) output
 // nodes.  The interior takes 32 x 8 (long rows: whole sectors), the shell
 // 16 x 16 (slabs are 8 to 20 nodes thick along j or k).
@@ -260,19 +212,6 @@ __global__ void __launch_bounds__(LayM<MASK>::NT, MASK == 7 ? 1 : 2) k_modal(Ste
     // (j, k, jk) of u and (const, j, k, jk) of v; z and minus its (j, k, jk)
     M3 w0[4], h0[3], v0[4], w1[4], h1[3], v1[4];
     float z0[4], zm0[3], z1[4], zm1[3];
-    auto sums4 = [](const M3 (&c)[4], M3 (&o)[4]) {
-        const M3 d0 = c[1] - c[0], d1 = c[3] - c[2], s0 = c[0] + c[1], s1 = c[2] + c[3];
-        o[0] = s0 + s1;
-        o[1] = d0 + d1;
-        o[2] = s1 - s0;
-        o[3] = d1 - d0;
-    };
-    auto sums3 = [](const M3 (&c)[4], M3 (&o)[3]) {
-        const M3 d0 = c[1] - c[0], d1 = c[3] - c[2], s0 = c[0] + c[1], s1 = c[2] + c[3];
-        o[0] = d0 + d1;
-        o[1] = s1 - s0;
-        o[2] = d1 - d0;
-    };
     // damped: the cell plane that the sums are for lies in a PML slab of z
     auto gather = [&](int slot, bool damped, M3 (&w)[4], M3 (&h)[3], M3 (&v)[4], float (&z)[4], float (&zm)[3]) {
         const float4* p = sN + slot * (2 * NP) + tx + NJ * ty;
@@ -290,9 +229,9 @@ __global__ void __launch_bounds__(LayM<MASK>::NT, MASK == 7 ? 1 : 2) k_modal(Ste
             H[c] = PML ? u : m_fma(A.dh2, V[c], A.hg1 * u);
             if (TER) z[c] = b.w;
         }
-        sums4(W, w);
-        sums3(H, h);
-        if (PML) sums4(V, v);
+        m_sums4(W, w);
+        m_sums3(H, h);
+        if (PML) m_sums4(V, v);
         if (TER) {
             // differences of z first: z is large against them
             const float d0 = z[0] - z[1], d1 = z[2] - z[3];

@@ -25,8 +25,7 @@
 // formed per cell corner).  MASK (bit d: axis d may be damped somewhere in
 // the box) compiles in the PML terms of those axes; which cells and nodes
 // are damped is decided per cell and node at run time, so a box may only
-// be given a MASK that covers every damped axis in it.  Boxes holding a
-// point source of the step are left to k_shell.
+// be given a MASK that covers every damped axis in it.
 #pragma once
 
 struct LaySl {
@@ -63,6 +62,21 @@ __global__ void __launch_bounds__(SJ * SK, 1) k_slab(StepArgs A) {
     const bool owncol = J >= j0 && J <= jm && K >= k0 && K <= km;
     const float dt = g.dt;
     float st_a = 0.f, st_v = 0.f, st_u = 0.f, st_w = 0.f;
+    // point sources (see k_interior)
+    __shared__ Inject lpot[kLocalInject], lmom[kLocalInject], lfrc[kLocalInject];
+    __shared__ int lcnt[3];
+    int npot = 0, nmom = 0, nfrc = 0;
+    if (A.ibox[0] <= jm && A.ibox[3] >= j0 - 1 && A.ibox[1] <= km && A.ibox[4] >= k0 - 1 && A.ibox[2] <= L1 &&
+        A.ibox[5] >= L0 - 1) {
+        gather_inject(A.pot, lpot, &lcnt[0], g, j0 - 1, jm, k0 - 1, km, L0 - 1, L1);
+        gather_inject(A.mom, lmom, &lcnt[1], g, j0 - 1, jm, k0 - 1, km, L0 - 1, L1);
+        gather_inject(A.force, lfrc, &lcnt[2], g, j0, jm, k0, km, L0, L1);
+        __syncthreads();
+        npot = lcnt[0];
+        nmom = lcnt[1];
+        nfrc = lcnt[2];
+    }
+    const bool scol = (npot != 0 || nmom != 0) && J >= A.ibox[0] && J <= A.ibox[3] && K >= A.ibox[1] && K <= A.ibox[4];
     // PML slabs of this thread's cell column (near, far) and node column
     const bool cnj = DJ && J <= g.i1pml[0], cfj = DJ && J >= g.i2pml[0] - 1;
     const bool cnk = DK && K <= g.i1pml[1], cfk = DK && K >= g.i2pml[1] - 1;
@@ -234,12 +248,26 @@ __global__ void __launch_bounds__(SJ * SK, 1) k_slab(StepArgs A) {
         eo[0] = sg[1][2] + sg[2][1];
         eo[1] = sg[0][2] + sg[2][0];
         eo[2] = sg[0][1] + sg[1][0];
+        const bool src = scol && l >= A.ibox[2] && l <= A.ibox[5];
+        float pd[3] = {0.f, 0.f, 0.f}, po[3] = {0.f, 0.f, 0.f};
+        if (src && npot != 0) {
+            apply_inject(lpot, npot, A.pot, g.idx(J, K, l), pd, po);
+#pragma unroll
+            for (int i = 0; i < 3; i++) { ed[i] = ed[i] + pd[i]; eo[i] = fmaf(2.0f, po[i], eo[i]); }
+        }
         {
             // (2 mu e + lam tr e) / V; the off-diagonal sums carry the 1/2
             const float r = cur[2], mur = cur[1] * r, m2r = mur + mur;
             const float s1r = (cur[0] * r) * (ed[0] + ed[1] + ed[2]);
 #pragma unroll
             for (int i = 0; i < 3; i++) { ed[i] = fmaf(m2r, ed[i], s1r); eo[i] = mur * eo[i]; }
+            if (src && nmom != 0) {
+#pragma unroll
+                for (int i = 0; i < 3; i++) pd[i] = po[i] = 0.f;
+                apply_inject(lmom, nmom, A.mom, g.idx(J, K, l), pd, po);
+#pragma unroll
+                for (int i = 0; i < 3; i++) { ed[i] = fmaf(pd[i], r, ed[i]); eo[i] = fmaf(po[i], r, eo[i]); }
+            }
         }
         if (A.stats && own)
             st_w = fmaxn(st_w, (ed[0] * ed[0] + ed[1] * ed[1] + ed[2] * ed[2]) + 2.0f * (eo[0] * eo[0] + eo[1] * eo[1] + eo[2] * eo[2]));
@@ -406,6 +434,18 @@ __global__ void __launch_bounds__(SJ * SK, 1) k_slab(StepArgs A) {
                 for (int ic = 0; ic < 3; ic++) fu[ic] = fu[ic] + fud[d][ic];
             }
         }
+        if (nfrc != 0) {
+            const Inject* E = nfrc >= 0 ? lfrc : A.force.e;
+            const int n = nfrc >= 0 ? nfrc : A.force.n;
+            for (int e = 0; e < n; e++)
+                if (E[e].idx == g.idx(jn, kn, l)) {
+                    const int c = E[e].comp;
+                    const float inc = E[e].inc;
+                    if (c == 0) fu[0] = fu[0] + inc;
+                    else if (c == 1) fu[1] = fu[1] + inc;
+                    else fu[2] = fu[2] + inc;
+                }
+        }
         finish_node<true>(A, g.idx(jn, kn, l), jn, kn, l, fu, cur[4], uv, dt, st_a, st_v, st_u);
     };
 
@@ -421,27 +461,26 @@ __global__ void __launch_bounds__(SJ * SK, 1) k_slab(StepArgs A) {
     fetch(L0 + 2);
     stat_load(L0 - 1, cur);
     uv_load(L0, uv);
-    cells(L0 - 1);
-    __syncthreads();  // cell plane L0-1 complete: its terms for node L0
-    nodes_fm(L0 - 1, false);
-    __syncthreads();  // one cell slot: read before cells(L0) overwrites it
-    stat_load(L0, cur);
+    // (one call of each phase, so that both are inlined)
 #pragma unroll 1
-    for (int l = L0; l <= L1; l++) {
+    for (int l = L0 - 1; l <= L1; l++) {
+        const bool first = l < L0;  // the cell plane below the first node plane
         cells(l);
         float nxt[5], nuv[6];
         stat_load(l + 1, nxt);
-        cp_async_wait_all();
+        if (!first) cp_async_wait_all();
         __syncthreads();  // cell plane l complete, staged plane l+2 landed
-        store((l + 2) % 3);
-        nodes_fm(l, true);
-        uv_load(l + 1, nuv);
+        if (!first) store((l + 2) % 3);
+        nodes_fm(l, !first);
+        if (!first) uv_load(l + 1, nuv);
         __syncthreads();  // ring slot l+2 complete, staging and the cell slot free
-        fetch(l + 3);
+        if (!first) {
+            fetch(l + 3);
+#pragma unroll
+            for (int i = 0; i < 6; i++) uv[i] = nuv[i];
+        }
 #pragma unroll
         for (int i = 0; i < 5; i++) cur[i] = nxt[i];
-#pragma unroll
-        for (int i = 0; i < 6; i++) uv[i] = nuv[i];
     }
     cp_async_wait_all();
     if (A.stats) {
