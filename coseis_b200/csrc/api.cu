@@ -241,6 +241,15 @@ static float read_max(Solver& s, int slot) {
     return f;
 }
 
+// the four statistics maxima of a fused step, one copy and one wait
+static void read_maxima(Solver& s) {
+    unsigned b[4];
+    SORD_CUDA(cudaMemcpyAsync(b, s.d.red, sizeof b, cudaMemcpyDeviceToHost, s.stream));
+    SORD_CUDA(cudaStreamSynchronize(s.stream));
+    float* to[4] = {&s.amax, &s.vmax, &s.umax, &s.wmax};
+    for (int i = 0; i < 4; i++) std::memcpy(to[i], b + i, sizeof(float));
+}
+
 static float norm_max(Solver& s, float* const w[3]) {
     int one[3] = {1, 1, 1};
     dev_vector_norm(s, s.d.s1, w, s.g.i1core, s.g.i2core, one);
@@ -343,12 +352,7 @@ void Solver::step(bool last_in_call) {
     }
     for (int i = 0; i < 3; i++) io("<>", kAcc[i], vol(*this, d.w1n[i]));
     io(">", "am2", vol(*this, d.s1));
-    if (st) {
-        amax = read_max(*this, 0);
-        vmax = read_max(*this, 1);
-        umax = read_max(*this, 2);
-        wmax = read_max(*this, 3);
-    }
+    if (st) read_maxima(*this);
     timers[1] = tio;
     timers[3] = clock_us() - t_step;
     stats();

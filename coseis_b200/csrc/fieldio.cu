@@ -111,8 +111,19 @@ __global__ void k_cube(float* f, Region R, const float* x0, const float* x1, con
     }
 }
 
-// '=>' gather of a strided region into one record
-__global__ void k_gather(const float* f, Region R, float* dst) {
+// '=>' gathers of strided regions into their records: one launch for the
+// ops of a field that fire together (24 single-node receivers of a step
+// took 24 launches of 3 us, now 3)
+struct GatherBatch {
+    static constexpr int kMost = 32;
+    int count;
+    Region R[kMost];
+    float* dst[kMost];
+    long long most;  // elements of the largest
+};
+__global__ void k_gather(const float* f, const __grid_constant__ GatherBatch b) {
+    const Region& R = b.R[blockIdx.y];
+    float* dst = b.dst[blockIdx.y];
     long long c0 = (R.i2[0] - R.i1[0]) / R.di[0] + 1, c1 = (R.i2[1] - R.i1[1]) / R.di[1] + 1, c2 = (R.i2[2] - R.i1[2]) / R.di[2] + 1;
     long long n = c0 * c1 * c2;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -878,7 +889,26 @@ static void disk_input(Solver& s, IoOp& io, FieldView f, int* i1, int* i2, int* 
     if (s.it == it2) { io.hbuf.clear(); io.op = "#"; }
 }
 
-static void field_io_op(Solver& s, size_t opi, FieldView f, ProbeBatch& batch) {
+// the outputs of one field_io call that are not launched yet
+struct OutBatch {
+    ProbeBatch probes;
+    GatherBatch gathers;
+};
+static void launch_outputs(Solver& s, const FieldView& f, OutBatch& b) {
+    if (b.probes.count) {
+        k_probe<<<1, 128, 0, s.stream>>>(f.p, b.probes);
+        FCHK(s);
+        b.probes.count = 0;
+    }
+    if (b.gathers.count) {
+        k_gather<<<dim3(gf(b.gathers.most), (unsigned)b.gathers.count), 256, 0, s.stream>>>(f.p, b.gathers);
+        FCHK(s);
+        b.gathers.count = 0;
+        b.gathers.most = 0;
+    }
+}
+
+static void field_io_op(Solver& s, size_t opi, FieldView f, OutBatch& out) {
     IoOp& io = s.ops[opi];
     const Geom& g = s.g;
     int i1[3], i2[3], i3[3], i4[3], di[3], m[4], n[4], o[4];
@@ -986,12 +1016,8 @@ static void field_io_op(Solver& s, size_t opi, FieldView f, ProbeBatch& batch) {
         float* dst = io.dbuf + (size_t)io.bufn * (io.ib - 1);
         if (io.op == ".>") {
             int id = probe_id(s, opi, io, f);
-            if (batch.count == 128) {
-                // flush a full batch before adding more
-                k_probe<<<1, 128, 0, s.stream>>>(f.p, batch);
-                FCHK(s);
-                batch.count = 0;
-            }
+            ProbeBatch& batch = out.probes;
+            if (batch.count == 128) launch_outputs(s, f, out);
             batch.probes = probe_table(s).dev;
             batch.id[batch.count] = id;
             batch.dst[batch.count] = dst;
@@ -1001,16 +1027,16 @@ static void field_io_op(Solver& s, size_t opi, FieldView f, ProbeBatch& batch) {
             for (int i = 0; i < 3; i++) { R.n[i] = f.n[i]; R.i1[i] = i1[i]; R.i2[i] = i2[i]; R.di[i] = di[i]; }
             R.vsy = g.sy; R.vsz = g.sz;
             if (nsp > 0) {
-                k_gather<<<gf(nsp), 256, 0, s.stream>>>(f.p, R, dst);
-                FCHK(s);
+                GatherBatch& batch = out.gathers;
+                if (batch.count == GatherBatch::kMost) launch_outputs(s, f, out);
+                batch.R[batch.count] = R;
+                batch.dst[batch.count] = dst;
+                batch.most = std::max(batch.most, (long long)nsp);
+                batch.count++;
             }
         } else throw SordError(SORD_E_PARAM, "bad i/o op");
         if (io.ib == io.nb || s.it == io.ii[3][1] || imod(s.it, s.prm.itio) == 0) {
-            if (batch.count) {
-                k_probe<<<1, 128, 0, s.stream>>>(f.p, batch);
-                FCHK(s);
-                batch.count = 0;
-            }
+            launch_outputs(s, f, out);
             int n3[3] = {n[0], n[1], n[2]}, m3[3] = {m[0], m[1], m[2]};
             flush_output(s, io, n3, m3);
         }
@@ -1022,9 +1048,11 @@ static void field_io_op(Solver& s, size_t opi, FieldView f, ProbeBatch& batch) {
 void field_io(Solver& s, const char* passes, const char* field, FieldView f) {
     for (const char* pp = passes; *pp; pp++) {
         char pass = *pp;
-        ProbeBatch batch;
-        batch.count = 0;
-        batch.probes = nullptr;
+        OutBatch batch;
+        batch.probes.count = 0;
+        batch.probes.probes = nullptr;
+        batch.gathers.count = 0;
+        batch.gathers.most = 0;
         bool any = false;
         for (size_t i = 0; i < s.ops.size(); i++) {
             if (applies(s, s.ops[i], field, pass, true)) any = true;
@@ -1037,10 +1065,7 @@ void field_io(Solver& s, const char* passes, const char* field, FieldView f) {
         // same exchanges
         if (pass == '<' && any && s.nparts > 1 && f.n[0] == s.g.nm[0] && f.n[1] == s.g.nm[1] && f.n[2] == s.g.nm[2])
             halo_exchange(s, &f.p, 1);
-        if (batch.count) {
-            k_probe<<<1, 128, 0, s.stream>>>(f.p, batch);
-            FCHK(s);
-        }
+        launch_outputs(s, f, batch);
     }
 }
 
