@@ -314,6 +314,11 @@ void Solver::step(bool last_in_call) {
         field_io(*this, passes, field, f);
         tio += clock_us() - t0;
     };
+    auto io_all = [&](const char* passes, const char* const* fields, float* const* p, int n) {
+        long long t0 = clock_us();
+        field_io(*this, passes, fields, p, n);
+        tio += clock_us() - t0;
+    };
     // leapfrog update of this step, unless the previous fused step did it
     // (for all nodes but the fault's, which fault_fold advances)
     tm = prm.tm0 + g.dt * (float)(it - 1);
@@ -323,9 +328,9 @@ void Solver::step(bool last_in_call) {
     } else if (g.ifn) {
         fault_fold(*this);
     }
-    for (int i = 0; i < 3; i++) io("<>", kVel[i], vol(*this, d.v[i]));
+    io_all("<>", kVel, d.v, 3);
     io(">", "vm2", vol(*this, d.s1));
-    for (int i = 0; i < 3; i++) io("<>", kDis[i], vol(*this, d.u[i]));
+    io_all("<>", kDis, d.u, 3);
     io(">", "um2", vol(*this, d.s1));
     if (g.ifn && !folded) fault_time_post(*this);
     std::vector<Inject> pot, mom, frc;
@@ -350,7 +355,7 @@ void Solver::step(bool last_in_call) {
         float* F[9] = {d.v[0], d.v[1], d.v[2], d.u[0], d.u[1], d.u[2], d.w1n[0], d.w1n[1], d.w1n[2]};
         halo_exchange(*this, F, 9);
     }
-    for (int i = 0; i < 3; i++) io("<>", kAcc[i], vol(*this, d.w1n[i]));
+    io_all("<>", kAcc, d.w1n, 3);
     io(">", "am2", vol(*this, d.s1));
     if (st) read_maxima(*this);
     timers[1] = tio;
@@ -373,15 +378,20 @@ void Solver::step_general(bool st) {
         field_io(*this, passes, field, f);
         tio += clock_us() - t0;
     };
+    auto io_all = [&](const char* passes, const char* const* fields, float* const* p, int n) {
+        long long t0 = clock_us();
+        field_io(*this, passes, fields, p, n);
+        tio += clock_us() - t0;
+    };
     // ---- step_time (time_integration.f90:6-115)
     if (G.ifn) fault_time_pre(*this);
     tm = prm.tm0 + G.dt * (float)(it - 1);
     const bool vin = any_pass(*this, kVel, 3, '<') || any_pass(*this, kDis, 3, '<');
     launch_time_update(*this, st && !vin);
-    for (int i = 0; i < 3; i++) io("<>", kVel[i], vol(*this, d.v[i]));
+    io_all("<>", kVel, d.v, 3);
     if (st) vmax = vin ? norm_max(*this, d.v) : read_max(*this, 1);
     io(">", "vm2", vol(*this, d.s1));
-    for (int i = 0; i < 3; i++) io("<>", kDis[i], vol(*this, d.u[i]));
+    io_all("<>", kDis, d.u, 3);
     if (st) umax = vin ? norm_max(*this, d.u) : read_max(*this, 2);
     io(">", "um2", vol(*this, d.s1));
     if (G.ifn) fault_time_post(*this);
@@ -394,7 +404,7 @@ void Solver::step_general(bool st) {
     if (fuse) {
         InjectList lp = upload_inject(*this, 0, pot), lm = upload_inject(*this, 1, mom);
         launch_stress(*this, lp, lm, true);
-        for (int i = 0; i < 6; i++) io("<>", kStr[i], vol(*this, sdso[i]));
+        io_all("<>", kStr, sdso, 6);
         if (st) wmax = read_max(*this, 3);
     } else {
         InjectList none{d.inj, 0};
@@ -402,12 +412,12 @@ void Solver::step_general(bool st) {
         pot.clear();
         mom.clear();
         if (prm.source == "potency") { finite_source_entries(*this, pot); launch_inject(*this, sdso, upload_inject(*this, 0, pot)); }
-        for (int i = 0; i < 6; i++) io("<>", kPot[i], vol(*this, sdso[i]));
+        io_all("<>", kPot, sdso, 6);
         launch_hooke(*this);
         if (prm.source == "moment") { finite_source_entries(*this, mom); launch_inject(*this, sdso, upload_inject(*this, 1, mom)); }
-        for (int i = 0; i < 6; i++) io("<>", kMom[i], vol(*this, sdso[i]));
+        io_all("<>", kMom, sdso, 6);
         launch_volume_scale(*this);
-        for (int i = 0; i < 6; i++) io("<>", kStr[i], vol(*this, sdso[i]));
+        io_all("<>", kStr, sdso, 6);
         if (st) {
             int one[3] = {1, 1, 1};
             dev_tensor_norm(*this, d.s1, d.sd, d.so, G.i1core, G.i2core, one);
@@ -437,7 +447,7 @@ void Solver::step_general(bool st) {
         for (int i = 0; i < 3; i++) io(">", kForce[i], vol(*this, d.w1n[i]));
         launch_mass(*this, st && !ain);
     }
-    for (int i = 0; i < 3; i++) io("<>", kAcc[i], vol(*this, d.w1n[i]));
+    io_all("<>", kAcc, d.w1n, 3);
     if (st) amax = ain ? norm_max(*this, d.w1n) : read_max(*this, 0);
     io(">", "am2", vol(*this, d.s1));
     timers[1] = tio;

@@ -112,17 +112,19 @@ __global__ void k_cube(float* f, Region R, const float* x0, const float* x1, con
 }
 
 // '=>' gathers of strided regions into their records: one launch for the
-// ops of a field that fire together (24 single-node receivers of a step
-// took 24 launches of 3 us, now 3)
+// ops that fire together, of one field or of the components of a vector or
+// tensor (24 single-node receivers of a step took 24 launches of 3 us, now 1)
 struct GatherBatch {
     static constexpr int kMost = 32;
     int count;
     Region R[kMost];
+    const float* src[kMost];
     float* dst[kMost];
     long long most;  // elements of the largest
 };
-__global__ void k_gather(const float* f, const __grid_constant__ GatherBatch b) {
+__global__ void k_gather(const __grid_constant__ GatherBatch b) {
     const Region& R = b.R[blockIdx.y];
+    const float* f = b.src[blockIdx.y];
     float* dst = b.dst[blockIdx.y];
     long long c0 = (R.i2[0] - R.i1[0]) / R.di[0] + 1, c1 = (R.i2[1] - R.i1[1]) / R.di[1] + 1, c2 = (R.i2[2] - R.i1[2]) / R.di[2] + 1;
     long long n = c0 * c1 * c2;
@@ -142,12 +144,14 @@ struct ProbeBatch {
     int count;
     const Probe* probes;  // device table (all probes)
     int id[128];          // probe ids firing now
+    const float* src[128];  // field of each
     float* dst[128];      // destination of each
 };
-__global__ void k_probe(const float* f, ProbeBatch b) {
+__global__ void k_probe(const __grid_constant__ ProbeBatch b) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.count) return;
     const Probe& P = b.probes[b.id[i]];
+    const float* f = b.src[i];
     float acc = 0.f;
     for (int t = 0; t < P.n; t++) acc = acc + f[P.idx[t]] * P.r[t];
     *b.dst[i] = acc;
@@ -889,19 +893,19 @@ static void disk_input(Solver& s, IoOp& io, FieldView f, int* i1, int* i2, int* 
     if (s.it == it2) { io.hbuf.clear(); io.op = "#"; }
 }
 
-// the outputs of one field_io call that are not launched yet
+// the outputs of one call that are not launched yet
 struct OutBatch {
     ProbeBatch probes;
     GatherBatch gathers;
 };
-static void launch_outputs(Solver& s, const FieldView& f, OutBatch& b) {
+static void launch_outputs(Solver& s, OutBatch& b) {
     if (b.probes.count) {
-        k_probe<<<1, 128, 0, s.stream>>>(f.p, b.probes);
+        k_probe<<<1, 128, 0, s.stream>>>(b.probes);
         FCHK(s);
         b.probes.count = 0;
     }
     if (b.gathers.count) {
-        k_gather<<<dim3(gf(b.gathers.most), (unsigned)b.gathers.count), 256, 0, s.stream>>>(f.p, b.gathers);
+        k_gather<<<dim3(gf(b.gathers.most), (unsigned)b.gathers.count), 256, 0, s.stream>>>(b.gathers);
         FCHK(s);
         b.gathers.count = 0;
         b.gathers.most = 0;
@@ -1017,9 +1021,10 @@ static void field_io_op(Solver& s, size_t opi, FieldView f, OutBatch& out) {
         if (io.op == ".>") {
             int id = probe_id(s, opi, io, f);
             ProbeBatch& batch = out.probes;
-            if (batch.count == 128) launch_outputs(s, f, out);
+            if (batch.count == 128) launch_outputs(s, out);
             batch.probes = probe_table(s).dev;
             batch.id[batch.count] = id;
+            batch.src[batch.count] = f.p;
             batch.dst[batch.count] = dst;
             batch.count++;
         } else if (io.op == "=>") {
@@ -1028,15 +1033,16 @@ static void field_io_op(Solver& s, size_t opi, FieldView f, OutBatch& out) {
             R.vsy = g.sy; R.vsz = g.sz;
             if (nsp > 0) {
                 GatherBatch& batch = out.gathers;
-                if (batch.count == GatherBatch::kMost) launch_outputs(s, f, out);
+                if (batch.count == GatherBatch::kMost) launch_outputs(s, out);
                 batch.R[batch.count] = R;
+                batch.src[batch.count] = f.p;
                 batch.dst[batch.count] = dst;
                 batch.most = std::max(batch.most, (long long)nsp);
                 batch.count++;
             }
         } else throw SordError(SORD_E_PARAM, "bad i/o op");
         if (io.ib == io.nb || s.it == io.ii[3][1] || imod(s.it, s.prm.itio) == 0) {
-            launch_outputs(s, f, out);
+            launch_outputs(s, out);
             int n3[3] = {n[0], n[1], n[2]}, m3[3] = {m[0], m[1], m[2]};
             flush_output(s, io, n3, m3);
         }
@@ -1045,28 +1051,47 @@ static void field_io_op(Solver& s, size_t opi, FieldView f, OutBatch& out) {
     throw SordError(SORD_E_PARAM, "bad i/o op");
 }
 
-void field_io(Solver& s, const char* passes, const char* field, FieldView f) {
-    for (const char* pp = passes; *pp; pp++) {
-        char pass = *pp;
-        OutBatch batch;
-        batch.probes.count = 0;
-        batch.probes.probes = nullptr;
-        batch.gathers.count = 0;
-        batch.gathers.most = 0;
-        bool any = false;
-        for (size_t i = 0; i < s.ops.size(); i++) {
-            if (applies(s, s.ops[i], field, pass, true)) any = true;
-            if (!applies(s, s.ops[i], field, pass)) continue;
-            field_io_op(s, i, f, batch);
-        }
-        // a partitioned run takes the halo planes of an input volume field
-        // from its neighbours (input_output.f90:218-238, 367 swap the staged
-        // values); `any` goes by the ops as read, so every part makes the
-        // same exchanges
-        if (pass == '<' && any && s.nparts > 1 && f.n[0] == s.g.nm[0] && f.n[1] == s.g.nm[1] && f.n[2] == s.g.nm[2])
-            halo_exchange(s, &f.p, 1);
-        launch_outputs(s, f, batch);
+// One pass of a field's hooks; outputs are left in `batch`.
+static void field_io_pass(Solver& s, char pass, const char* field, FieldView f, OutBatch& batch) {
+    bool any = false;
+    for (size_t i = 0; i < s.ops.size(); i++) {
+        if (applies(s, s.ops[i], field, pass, true)) any = true;
+        if (!applies(s, s.ops[i], field, pass)) continue;
+        if (pass == '<') launch_outputs(s, batch);  // what they read is still as it was
+        field_io_op(s, i, f, batch);
     }
+    // a partitioned run takes the halo planes of an input volume field
+    // from its neighbours (input_output.f90:218-238, 367 swap the staged
+    // values); `any` goes by the ops as read, so every part makes the
+    // same exchanges
+    if (pass == '<' && any && s.nparts > 1 && f.n[0] == s.g.nm[0] && f.n[1] == s.g.nm[1] && f.n[2] == s.g.nm[2])
+        halo_exchange(s, &f.p, 1);
+}
+
+// The hooks of one field, or of n volume fields that have the same hook in turn: the
+// outputs of all of them that fire now are launched together.
+void field_io(Solver& s, const char* passes, const char* const* fields, float* const* p, int n) {
+    OutBatch batch;
+    batch.probes.count = 0;
+    batch.probes.probes = nullptr;
+    batch.gathers.count = 0;
+    batch.gathers.most = 0;
+    for (int c = 0; c < n; c++) {
+        FieldView f;
+        f.p = p[c];
+        for (int i = 0; i < 3; i++) f.n[i] = s.g.nm[i];
+        for (const char* pp = passes; *pp; pp++) field_io_pass(s, *pp, fields[c], f, batch);
+    }
+    launch_outputs(s, batch);
+}
+void field_io(Solver& s, const char* passes, const char* field, FieldView f) {
+    OutBatch batch;
+    batch.probes.count = 0;
+    batch.probes.probes = nullptr;
+    batch.gathers.count = 0;
+    batch.gathers.most = 0;
+    for (const char* pp = passes; *pp; pp++) field_io_pass(s, *pp, field, f, batch);
+    launch_outputs(s, batch);
 }
 
 void field_io_flush_all(Solver& s) { (void)s; }

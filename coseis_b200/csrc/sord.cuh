@@ -262,6 +262,7 @@ struct FieldView {
     int n[3];
 };
 void field_io(Solver& s, const char* passes, const char* field, FieldView f);
+void field_io(Solver& s, const char* passes, const char* const* fields, float* const* p, int n);
 void field_io_flush_all(Solver& s);
 InjectList upload_inject(Solver& s, int slot, const std::vector<Inject>& e);  // through the slot's ring (api.cu)
 void halo_exchange(Solver& s, float* const* fields, int nf);  // halo planes along l from the neighbouring parts
