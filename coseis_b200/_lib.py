@@ -17,7 +17,7 @@ SYMBOLS = [
     'sord_last_error', 'sord_error_string', 'sord_destroy',
     'sord_vector_max_noalloc', 'sord_run_ensemble', 'sord_adjoint_forward', 'sord_adjoint_backward',
     'sord_set_arithmetic', 'sord_get_arithmetic', 'sord_trim_memory', 'sord_adjoint_source_gradients',
-    'sord_adjoint_forward_binomial', 'sord_adjoint_binomial_cost',
+    'sord_adjoint_forward_binomial', 'sord_adjoint_material', 'sord_adjoint_binomial_cost',
     'sord_set_field', 'sord_create_part',
 ]
 
@@ -108,6 +108,8 @@ def load():
     DP = ctypes.POINTER(ctypes.c_double)
     lib.sord_adjoint_source_gradients.argtypes = [P, DP, DP, ctypes.c_int]
     lib.sord_adjoint_source_gradients.restype = ctypes.c_int
+    lib.sord_adjoint_material.argtypes = [P, DP, DP, DP, DP, DP, DP, DP]
+    lib.sord_adjoint_material.restype = ctypes.c_int
     lib.sord_vector_max_noalloc.argtypes = [P, P, P, IP, IP, IP, P, P]
     lib.sord_vector_max_noalloc.restype = ctypes.c_int
     _lib = lib
@@ -245,6 +247,23 @@ class Solver(object):
         res['position'] = gx[:3 * nmoment].reshape(nmoment, 3)  # dL/dx of each moment op (per metre)
         res['delay'] = gt[:nmoment]                             # dL/dt0 of each moment op (per second)
         return res
+
+    def adjoint_material(self, rho, vp, vs, delta):
+        """After adjoint_backward: its gradients with respect to rho, vp and
+        vs, the cell fields' values given ([j, k, l], any float type), as
+        float64 arrays; adjoint.material_chain on the device."""
+        import numpy as np
+        nn, it, nt = self.info()
+        shape = tuple(x - 1 for x in nn)
+        arrs = [np.ascontiguousarray(a, np.float64) for a in (rho, vp, vs)]
+        if any(a.shape != shape for a in arrs):
+            raise ValueError('cells are %s' % (shape,))
+        out = [np.empty(shape, np.float64) for _ in range(3)]
+        DP = ctypes.POINTER(ctypes.c_double)
+        d = (ctypes.c_double * 3)(*[float(x) for x in delta[:3]])
+        _check(load().sord_adjoint_material(self._h, *[a.ctypes.data_as(DP) for a in arrs], d,
+                                            *[a.ctypes.data_as(DP) for a in out]), self._h)
+        return out
 
     def run(self):
         _check(load().sord_run(self._h), self._h)

@@ -1300,16 +1300,11 @@ void adjoint_backward(Solver& s, int nrec, const char* const* files, const float
     SORD_CUDA(cudaEventElapsedTime(&ms, s.ev0, s.ev1));
     s.last_step_ms = ms;
     // gradients of the real cells and nodes, global order (j fastest)
-    std::vector<float> buf(nv);
-    auto out = [&](const float* d, float* host, bool cell) {
+    auto out = [&](float* d, float* host, bool cell) {
         if (!host) return;
-        SORD_CUDA(cudaMemcpyAsync(buf.data(), d, sizeof(float) * nv, cudaMemcpyDeviceToHost, s.stream));
-        SORD_CUDA(cudaStreamSynchronize(s.stream));
-        const int e0 = s.g.nn[0] - (cell ? 1 : 0), e1 = s.g.nn[1] - (cell ? 1 : 0), e2 = s.g.nn[2] - (cell ? 1 : 0);
-        size_t o = 0;
-        for (int l = 1; l <= e2; l++)
-            for (int k = 1; k <= e1; k++)
-                for (int j = 1; j <= e0; j++) host[o++] = buf[g.idx(j - g.nnoff[0], k - g.nnoff[1], l - g.nnoff[2])];
+        int c[3];
+        for (int i = 0; i < 3; i++) c[i] = s.g.nn[i] - (cell ? 1 : 0);
+        core_transfer(s, d, host, nullptr, c);
     };
     out(A->glam, glam, true);
     out(A->gmu, gmu, true);
@@ -1321,6 +1316,100 @@ void adjoint_backward(Solver& s, int nrec, const char* const* files, const float
     SORD_CUDA(cudaStreamSynchronize(s.stream));
     if (gmom && nmom > 0) std::copy(A->gsrc.begin(), A->gsrc.begin() + nmom, gmom);
     A->gsrc.erase(A->gsrc.begin(), A->gsrc.begin() + std::max(nmom, 1));
+}
+
+// Chain rule of the material setup at a cell: (dlam, dmu, dyy) and the dmr of
+// its eight nodes -> (drho, dvp, dvs), in the order of operations of
+// adjoint.material_chain, so that the two agree to the last bit.  Rows of j
+// are slowest, as the arrays come from the caller; rho has the rows on both
+// sides of this slab too, which the nodal masses read.  Bound by the copies of
+// the six arrays over the bus; a node's mass is formed again by each of its
+// cells (64 cached loads) rather than kept.
+struct MaterialArgs {
+    Geom g;
+    const float *glam, *gmu, *gyy, *gmr;
+    const double *rho, *vp, *vs;  // rho from row r0, the others from row j0
+    double *grho, *gvp, *gvs;
+    int c[3], j0, r0;
+    long long n;
+    double s, V;
+};
+__global__ void __launch_bounds__(256) k_adj_material(MaterialArgs A) {
+    const Geom& g = A.g;
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t >= A.n) return;
+    const int l = (int)(t % A.c[2]), k = (int)((t / A.c[2]) % A.c[1]), j = A.j0 + (int)(t / ((long long)A.c[1] * A.c[2]));
+    auto at = [&](int J, int K, int L) { return g.idx(J + 1 - g.nnoff[0], K + 1 - g.nnoff[1], L + 1 - g.nnoff[2]); };
+    auto row = [&](int J, int K, int L) { return A.rho[((long long)(J - A.r0) * A.c[1] + K) * A.c[2] + L]; };
+    const double rho = row(j, k, l), vp = A.vp[t], vs = A.vs[t];
+    const double mu = rho * vs * vs, lam = rho * vp * vp - 2.0 * mu, r = lam + 2.0 * mu;
+    const double dl = r != 0 ? A.s * mu * mu / (r * r) : 0.0;
+    const double dm = r != 0 ? A.s * (lam * lam + 2.0 * lam * mu + 2.0 * mu * mu) / (r * r) : 0.0;
+    const long long q = at(j, k, l);
+    const double gy = A.gyy[q];
+    const double gl = (double)A.glam[q] + gy * dl, gm = (double)A.gmu[q] + gy * dm;
+    double gr = gl * (vp * vp - 2.0 * vs * vs) + gm * vs * vs;
+    A.gvp[t] = gl * 2.0 * rho * vp;
+    A.gvs[t] = gl * (-4.0 * rho * vs) + gm * 2.0 * rho * vs;
+    // nodal mass: mr(n) = 1 / (sum over the 8 cells around n of rho V / 8)
+    for (int d = 0; d < 8; d++) {
+        const int J = j + (d >> 2), K = k + ((d >> 1) & 1), L = l + (d & 1);
+        double S = 0.0;
+        for (int e = 0; e < 8; e++) {
+            const int a = J - (e >> 2), b = K - ((e >> 1) & 1), c = L - (e & 1);
+            if (a >= 0 && a < A.c[0] && b >= 0 && b < A.c[1] && c >= 0 && c < A.c[2]) S = S + row(a, b, c) * A.V;
+        }
+        const double mr = S != 0 ? 8.0 / S : 0.0;
+        gr = gr + (double)A.gmr[at(J, K, L)] * (-mr * mr) * 0.125 * A.V;
+    }
+    A.grho[t] = gr;
+}
+
+// Gradients of the last backward pass with respect to rho, vp and vs, whose
+// values (nn - 1 per axis, [j][k][l]) the caller gives; slabs of rows j.
+void adjoint_material(Solver& s, const double* rho, const double* vp, const double* vs, const double delta[3], double* grho,
+                      double* gvp, double* gvs) {
+    AdjointState* A = s.adj;
+    if (!A || A->gsrc.empty()) throw SordError(SORD_E_STATE, "adjoint: no backward pass recorded");
+    MaterialArgs M;
+    M.g = s.g;
+    M.glam = A->glam; M.gmu = A->gmu; M.gyy = A->gyy; M.gmr = A->gmr;
+    for (int i = 0; i < 3; i++) M.c[i] = s.g.nn[i] - 1;
+    if (M.c[0] < 1 || M.c[1] < 1 || M.c[2] < 1) throw SordError(SORD_E_PARAM, "adjoint: no cells");
+    M.s = std::sqrt((delta[0] * delta[0] + delta[1] * delta[1] + delta[2] * delta[2]) / 3.0) / 12.0;
+    M.V = delta[0] * delta[1] * delta[2];
+    const size_t plane = (size_t)M.c[1] * M.c[2];
+    const int rows = (int)std::min<size_t>((size_t)M.c[0], std::max<size_t>(1, ((size_t)4 << 20) / plane));
+    struct Mem {
+        Solver& s;
+        void* p = nullptr;
+        ~Mem() { dev_free(s, p); }
+    } mem{s};
+    if (dev_malloc(s, &mem.p, sizeof(double) * plane * (6 * (size_t)rows + 2)) != cudaSuccess) {
+        cudaGetLastError();
+        mem.p = nullptr;
+        throw SordError(SORD_E_NOMEM, "adjoint: cannot allocate device memory");
+    }
+    double* d = (double*)mem.p;
+    const size_t slab = plane * rows;
+    double *drho = d + 5 * slab, *dvp = d, *dvs = d + slab;
+    M.vp = dvp; M.vs = dvs; M.rho = drho;
+    M.grho = d + 2 * slab; M.gvp = d + 3 * slab; M.gvs = d + 4 * slab;
+    for (int j0 = 0; j0 < M.c[0]; j0 += rows) {
+        const int m = std::min(rows, M.c[0] - j0), r0 = std::max(j0 - 1, 0), r1 = std::min(j0 + m + 1, M.c[0]);
+        const size_t at = plane * j0, bytes = sizeof(double) * plane * m;
+        M.j0 = j0; M.r0 = r0; M.n = (long long)(plane * m);
+        SORD_CUDA(cudaMemcpyAsync(drho, rho + plane * r0, sizeof(double) * plane * (r1 - r0), cudaMemcpyHostToDevice, s.stream));
+        SORD_CUDA(cudaMemcpyAsync(dvp, vp + at, bytes, cudaMemcpyHostToDevice, s.stream));
+        SORD_CUDA(cudaMemcpyAsync(dvs, vs + at, bytes, cudaMemcpyHostToDevice, s.stream));
+        k_adj_material<<<(unsigned)((M.n + 255) / 256), 256, 0, s.stream>>>(M);
+        s.launches++;
+        SORD_CUDA(cudaGetLastError());
+        SORD_CUDA(cudaMemcpyAsync(grho + at, M.grho, bytes, cudaMemcpyDeviceToHost, s.stream));
+        SORD_CUDA(cudaMemcpyAsync(gvp + at, M.gvp, bytes, cudaMemcpyDeviceToHost, s.stream));
+        SORD_CUDA(cudaMemcpyAsync(gvs + at, M.gvs, bytes, cudaMemcpyDeviceToHost, s.stream));
+    }
+    SORD_CUDA(cudaStreamSynchronize(s.stream));
 }
 
 // Delay (t0) and position gradients of each '.' moment op from the last

@@ -709,7 +709,7 @@ __global__ void k_core(float* f, float* buf, Geom g, int n0, int n1, int l1, lon
 
 // Core region of field f (c nodes or cells per axis) to host memory (out) or
 // from it (in), in chunks of planes through two pinned buffers.
-static void core_transfer(Solver& s, float* f, float* out, const float* in, const int* c) {
+void core_transfer(Solver& s, float* f, float* out, const float* in, const int* c) {
     const size_t plane = (size_t)c[0] * c[1];
     if (plane == 0 || c[2] == 0) return;
     const int step = (int)std::max<size_t>(1, std::min<size_t>((size_t)c[2], ((size_t)4 << 20) / plane));
@@ -892,6 +892,19 @@ int sord_adjoint_source_gradients(sord_handle* h, double* grad_x0, double* grad_
     if (!h || nmoment < 0) return SORD_E_PARAM;
     try {
         adjoint_source_gradients(h->s, grad_x0, grad_t0, nmoment);
+    } catch (const std::exception& e) {
+        return fail(h, e);
+    }
+    return SORD_OK;
+}
+
+int sord_adjoint_material(sord_handle* h, const double* rho, const double* vp, const double* vs, const double* delta,
+                          double* grad_rho, double* grad_vp, double* grad_vs) {
+    if (!h || !rho || !vp || !vs || !delta || !grad_rho || !grad_vp || !grad_vs) return SORD_E_PARAM;
+    Solver& s = h->s;
+    try {
+        SORD_CUDA(cudaSetDevice(s.device));
+        adjoint_material(s, rho, vp, vs, delta, grad_rho, grad_vp, grad_vs);
     } catch (const std::exception& e) {
         return fail(h, e);
     }

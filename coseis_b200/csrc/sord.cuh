@@ -389,6 +389,9 @@ void adjoint_checkpoint(Solver& s);
 void adjoint_backward(Solver& s, int nrec, const char* const* files, const float* const* dtrace, const int* ntrace,
                       float* glam, float* gmu, float* gyy, float* gmr, double* gmom, int nmom);
 void adjoint_source_gradients(Solver& s, double* gx, double* gt, int nmom);
+void adjoint_material(Solver& s, const double* rho, const double* vp, const double* vs, const double delta[3], double* grho,
+                      double* gvp, double* gvs);
+void core_transfer(Solver& s, float* f, float* out, const float* in, const int* c);  // core region to or from host memory
 void mem_attach(int device);
 void mem_detach(int device);
 void mem_trim(int device);

@@ -170,6 +170,14 @@ int sord_trim_memory(int device);
  * sord_adjoint_backward. */
 int sord_adjoint_source_gradients(sord_handle* h, double* grad_x0, double* grad_t0, int nmoment);
 
+/* After sord_adjoint_backward: its gradients carried through the material
+ * setup (material_model.f90:65-76, 120-134; material_resample.f90:16-18) to
+ * the cell fields rho, vp and vs.  All six arrays are host doubles of nn-1
+ * values per axis indexed [j][k][l] (l fastest); delta holds the three node
+ * spacings.  Material limits are not differentiated. */
+int sord_adjoint_material(sord_handle* h, const double* rho, const double* vp, const double* vs, const double* delta,
+                          double* grad_rho, double* grad_vp, double* grad_vs);
+
 /* Copy a node or cell volume field to host memory (core region only, j
  * fastest; nn or nn-1 values per axis).  Names: vx vy vz ux uy uz ax ay az
  * (nodes; `a` holds the last acceleration) and lam mu yy vc (cells).
