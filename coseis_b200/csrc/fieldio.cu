@@ -897,6 +897,14 @@ static void disk_input(Solver& s, IoOp& io, FieldView f, int* i1, int* i2, int* 
 struct OutBatch {
     ProbeBatch probes;
     GatherBatch gathers;
+    struct Full { size_t op; int n[3], m[3]; };
+    std::vector<Full> full;  // ops whose buffer goes to its file afterwards
+    OutBatch() {
+        probes.count = 0;
+        probes.probes = nullptr;
+        gathers.count = 0;
+        gathers.most = 0;
+    }
 };
 static void launch_outputs(Solver& s, OutBatch& b) {
     if (b.probes.count) {
@@ -1042,13 +1050,16 @@ static void field_io_op(Solver& s, size_t opi, FieldView f, OutBatch& out) {
             }
         } else throw SordError(SORD_E_PARAM, "bad i/o op");
         if (io.ib == io.nb || s.it == io.ii[3][1] || imod(s.it, s.prm.itio) == 0) {
-            launch_outputs(s, out);
-            int n3[3] = {n[0], n[1], n[2]}, m3[3] = {m[0], m[1], m[2]};
-            flush_output(s, io, n3, m3);
+            out.full.push_back(OutBatch::Full{opi, {n[0], n[1], n[2]}, {m[0], m[1], m[2]}});
         }
         return;
     }
     throw SordError(SORD_E_PARAM, "bad i/o op");
+}
+
+static void finish_outputs(Solver& s, OutBatch& batch) {
+    launch_outputs(s, batch);
+    for (OutBatch::Full& f : batch.full) flush_output(s, s.ops[f.op], f.n, f.m);
 }
 
 // One pass of a field's hooks; outputs are left in `batch`.
@@ -1072,26 +1083,18 @@ static void field_io_pass(Solver& s, char pass, const char* field, FieldView f, 
 // outputs of all of them that fire now are launched together.
 void field_io(Solver& s, const char* passes, const char* const* fields, float* const* p, int n) {
     OutBatch batch;
-    batch.probes.count = 0;
-    batch.probes.probes = nullptr;
-    batch.gathers.count = 0;
-    batch.gathers.most = 0;
     for (int c = 0; c < n; c++) {
         FieldView f;
         f.p = p[c];
         for (int i = 0; i < 3; i++) f.n[i] = s.g.nm[i];
         for (const char* pp = passes; *pp; pp++) field_io_pass(s, *pp, fields[c], f, batch);
     }
-    launch_outputs(s, batch);
+    finish_outputs(s, batch);
 }
 void field_io(Solver& s, const char* passes, const char* field, FieldView f) {
     OutBatch batch;
-    batch.probes.count = 0;
-    batch.probes.probes = nullptr;
-    batch.gathers.count = 0;
-    batch.gathers.most = 0;
     for (const char* pp = passes; *pp; pp++) field_io_pass(s, *pp, field, f, batch);
-    launch_outputs(s, batch);
+    finish_outputs(s, batch);
 }
 
 void field_io_flush_all(Solver& s) { (void)s; }
