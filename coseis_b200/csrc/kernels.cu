@@ -154,6 +154,25 @@ __global__ void __launch_bounds__(256) k_stress(StressArgs A) {
 #pragma unroll
             for (int a = 0; a < 3; a++) brackets_nc(X, a, B[a]);
         }
+        // the memories of the damped directions, loaded before the first of
+        // them is stored: a load after a store waits for it in turn, up to
+        // nine times in a corner (52 us on 96 x 80 x 72 nodes with ten PML
+        // planes, now 47; bound by the latency of the loads, with two blocks
+        // per SM.  A third block, at 80 registers, spills and gained nothing)
+        float G0[3][3];
+        if (anyS) {
+#pragma unroll
+            for (int id = 0; id < 3; id++) {
+                const int c = id == 0 ? j : id == 1 ? k : l;
+                const int side = nearS[id] ? id : 3 + id;
+#pragma unroll
+                for (int ic = 0; ic < 3; ic++)
+                    G0[id][ic] = nearS[id] || farS[id]
+                                     ? A.sl.g[side][slab_index(g, id, A.sl.tg[side], nearS[id] ? c - g.i1cell[id] : g.i2cell[id] - c,
+                                                               j, k, l, ic)]
+                                     : 0.f;
+            }
+        }
         float ed[3], eo[3];
         const float h = g.h;
 #pragma unroll
@@ -179,14 +198,14 @@ __global__ void __launch_bounds__(256) k_stress(StressArgs A) {
                         int p = c + g.nnoff[id];
                         int ii = c - g.i1cell[id];
                         float* G = A.sl.g[id] + slab_index(g, id, A.sl.tg[id], ii, j, k, l, ic);
-                        s = A.pmlc[3 * g.npml + p - 1] * raw + A.pmlc[2 * g.npml + p - 1] * *G;
+                        s = A.pmlc[3 * g.npml + p - 1] * raw + A.pmlc[2 * g.npml + p - 1] * G0[id][ic];
                         *G = s;
                     }
                     if (farS[id]) {
                         int p = g.nn[id] - c - g.nnoff[id];
                         int ii = g.i2cell[id] - c;
                         float* G = A.sl.g[3 + id] + slab_index(g, id, A.sl.tg[3 + id], ii, j, k, l, ic);
-                        s = A.pmlc[3 * g.npml + p - 1] * raw + A.pmlc[2 * g.npml + p - 1] * *G;
+                        s = A.pmlc[3 * g.npml + p - 1] * raw + A.pmlc[2 * g.npml + p - 1] * (nearS[id] ? *G : G0[id][ic]);
                         *G = s;
                     }
                 } else if (anyS) {
