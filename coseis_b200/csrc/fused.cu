@@ -1146,16 +1146,25 @@ void fused_free(Solver& s) {
 // Planes per block.  Each block streams its column through the planes, so
 // a small mesh is cut into shorter plane ranges until both kernels have
 // about kWaveBlocks blocks per SM; a range starts with a prologue of about
-// two planes, so it is kept at kMinPlanes planes or more; in fast
-// arithmetic, whose prologue is one cell plane, down to kFewPlanes where a
-// launch would leave SMs without a block.
+// two planes, so it is kept at kMinPlanes planes or more, and down to
+// kFewPlanes only where the launch does not fill the chip: below a block per
+// SM in fast arithmetic, below the two that fit in reference order, whose
+// planes take longer.  61^3 nodes in reference order, 200 steps: eight
+// planes 32.6 ms, four 27.5; one step of 24^3 275 and 250 us.  (Four below
+// 592 blocks: 256 x 256 x 128 nodes 1 % slower; four below two blocks per SM
+// in fast arithmetic: 203 x 149 x 97 nodes 2 % slower; three planes: no
+// faster on 61^3.)
 static constexpr int kItemPlanes = 96;
 static constexpr int kMinPlanes = 8;
 static constexpr int kFewPlanes = 4;
 static constexpr int kWaveBlocks = 4;
 
-// shell items covering node box [j1, j2] x [k1, k2] x [l1, l2]
+// shell items covering node box [j1, j2] x [k1, k2] x [l1, l2], of at most
+// ipl planes and as even as they can be: a launch lasts as long as its
+// longest item
 static void push_box(std::vector<int>& v, int ipl, int j1, int j2, int k1, int k2, int l1, int l2) {
+    const int planes = l2 - l1 + 1, parts = (planes + ipl - 1) / ipl;
+    ipl = parts > 0 ? (planes + parts - 1) / parts : 1;
     for (int a = l1; a <= l2; a += ipl)
         for (int k = k1; k <= k2; k += SK - 1)
             for (int j = j1; j <= j2; j += SJ - 1) {
@@ -1175,8 +1184,8 @@ static FusedPlan& fused_plan(Solver& s) {
     FusedPlan* P = new FusedPlan();
     s.fplan = P;
     P->arith = s.arith;
-    // shortest plane range where a launch has less than a block per SM
-    const int few = s.arith ? kFewPlanes : kMinPlanes;
+    // shortest plane range of a launch that does not fill the chip
+    const int few = kFewPlanes;
     const Geom& g = s.g;
     // Node c along axis d is interior when it is outside the PML and each
     // adjacent cell is either a real cell outside the PML or a cell outside
@@ -1243,8 +1252,8 @@ static FusedPlan& fused_plan(Solver& s) {
     };
     // Planes per item, per class: each class is one launch (on its own
     // stream), so its items are cut as long as the launch still has about
-    // kWaveBlocks blocks per SM, and no shorter than kMinPlanes (an item
-    // starts with a prologue of about two planes).
+    // kWaveBlocks blocks per SM, and no shorter than kMinPlanes, or than
+    // kFewPlanes where less is resident than could be.
     std::vector<int> rcls;
     for (const RegionBox& r : rb) rcls.push_back(klass(r.lo, r.hi));
     int iplc[4];
@@ -1259,7 +1268,7 @@ static FusedPlan& fused_plan(Solver& s) {
         };
         int ipl = kItemPlanes;
         while (ipl > kMinPlanes && count(ipl) < want) ipl = std::max(kMinPlanes, ipl * 2 / 3);
-        while (ipl > few && count(ipl) < sms) ipl = std::max(few, ipl * 2 / 3);
+        while (ipl > few && count(ipl) < (s.arith ? sms : 2 * sms)) ipl = std::max(few, ipl * 2 / 3);
         iplc[c] = ipl;
     }
     // boxes by their own class (a range of planes may miss the PML of z)
