@@ -1075,8 +1075,19 @@ void adjoint_backward(Solver& s, int nrec, const char* const* files, const float
     K.nbx = std::max(1, (K.box2[0] - K.box1[0] + AJ - 1) / (AJ - 1));
     const int nby = std::max(1, (K.box2[1] - K.box1[1] + AK - 1) / (AK - 1));
     const int planes = std::max(1, K.box2[2] - K.box1[2] + 1);
-    const int nsg = std::max(1, std::min((4 * sms + K.nbx * nby - 1) / (K.nbx * nby), planes / 8));
-    K.segl = (planes + nsg - 1) / nsg;
+    // the split along l that takes the fewest plane times: rounds of two
+    // blocks per SM, each its planes and a prologue of about two (eight planes
+    // or more at any size: 53 us on 44 x 40 x 36 nodes, 60 blocks, and now 27)
+    double best = 0;
+    for (int n = 1; n <= std::max(1, planes / 3); n++) {
+        const int len = (planes + n - 1) / n;
+        const long long blocks = (long long)K.nbx * nby * ((planes + len - 1) / len);
+        const double t = (double)((blocks + 2 * sms - 1) / (2 * sms)) * (len + 2);
+        if (n == 1 || t < best) {
+            best = t;
+            K.segl = len;
+        }
+    }
     const dim3 agrid((unsigned)(K.nbx * nby), (unsigned)((planes + K.segl - 1) / K.segl));
     smem_limit((const void*)k_adj_step, (int)kAdjSmem);
     // PML runs: the two-pass step over cells and nodes
@@ -1131,13 +1142,16 @@ void adjoint_backward(Solver& s, int nrec, const char* const* files, const float
     // overlaps the adjoint pass over segment k.
     struct Streams {
         cudaStream_t as = nullptr;
-        cudaEvent_t ev[5] = {};  // rec_done[2], adj_done[2], start
+        cudaStream_t side = nullptr;  // k_adj_step of a run with PML
+        cudaEvent_t ev[7] = {};  // rec_done[2], adj_done[2], start, fork, join
         ~Streams() {
             for (auto e : ev) if (e) cudaEventDestroy(e);
             if (as) cudaStreamDestroy(as);
+            if (side) cudaStreamDestroy(side);
         }
     } S;
     SORD_CUDA(cudaStreamCreateWithFlags(&S.as, cudaStreamNonBlocking));
+    SORD_CUDA(cudaStreamCreateWithFlags(&S.side, cudaStreamNonBlocking));
     for (auto& e : S.ev) SORD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     cudaEvent_t* rec_done = S.ev;
     cudaEvent_t* adj_done = S.ev + 2;
@@ -1159,15 +1173,20 @@ void adjoint_backward(Solver& s, int nrec, const char* const* files, const float
             }
             for (int i = 0; i < 6; i++) KP.gf[i] = st + A->gofs[i];
             // the fused kernel on the nodes away from the PML, the two
-            // passes on the rest (they write disjoint nodes and cells)
+            // passes on the rest (they write disjoint nodes and cells, so
+            // the two run side by side; neither fills the chip)
             if (fused_box) {
-                if (nme > 0) k_adj_moment<<<(nme + 31) / 32, 256, 0, as>>>(K, A->mom + moff[n], nme, A->gmom);
-                k_adj_step<<<agrid, dim3(AJ, AK), kAdjSmem, as>>>(K);
+                SORD_CUDA(cudaEventRecord(S.ev[5], as));
+                SORD_CUDA(cudaStreamWaitEvent(S.side, S.ev[5], 0));
+                if (nme > 0) k_adj_moment<<<(nme + 31) / 32, 256, 0, S.side>>>(K, A->mom + moff[n], nme, A->gmom);
+                k_adj_step<<<agrid, dim3(AJ, AK), kAdjSmem, S.side>>>(K);
+                SORD_CUDA(cudaEventRecord(S.ev[6], S.side));
                 s.launches += 1 + (nme > 0 ? 1 : 0);
             }
             k_adjp_cells<<<pcgrid, pblock, 0, as>>>(KP);
             if (nme > 0) k_adjp_moment<<<1, 128, 0, as>>>(K, A->cs + (size_t)CS_SIG * nv, A->mom + moff[n], nme, A->gmom);
             k_adjp_nodes<<<pngrid, pblock, 0, as>>>(KP);
+            if (fused_box) SORD_CUDA(cudaStreamWaitEvent(as, S.ev[6], 0));
             s.launches++;
         } else {
             if (nme > 0) k_adj_moment<<<(nme + 31) / 32, 256, 0, as>>>(K, A->mom + moff[n], nme, A->gmom);
