@@ -367,9 +367,9 @@ void Solver::step(bool last_in_call) {
 // time_integration.f90, stress.f90 and acceleration.f90 in place.
 void Solver::step_general(bool st) {
     Geom& G = g;
-    if (d.statics_made) {
+    if (d.statics_there) {
         // the stress fields take the statics' place; off the mesh they are zero
-        d.statics_made = false;
+        d.statics_there = d.statics_valid = false;
         for (float* f : {d.sd[0], d.sd[1], d.sd[2], d.so[0]}) dev_fill(*this, f, G.nv, 0.f);
     }
     long long tio = 0;
@@ -1025,7 +1025,7 @@ int sord_set_field(sord_handle* h, const char* name, const float* host, size_t n
         if (n != need) throw SordError(SORD_E_PARAM, "host array has " + std::to_string(n) + " values, the field " +
                                                      std::to_string(need));
         core_transfer(s, dst, nullptr, host, c);
-        if (cell) s.d.statics_made = false;
+        if (cell) s.d.statics_valid = false;
     } catch (const std::exception& e) {
         return fail(h, e);
     }

@@ -1414,11 +1414,11 @@ static void launch_class(Solver& s, const StepArgs& A, int cls, unsigned n, cuda
 static const float4* modal_statics(Solver& s) {
     Device& d = s.d;
     float4* sta = (float4*)d.sd[0];
-    if (!d.statics_made) {
+    if (!d.statics_valid) {
         k_statics<<<div_up(std::min(s.g.nv, 148LL * 64 * 256), 256), 256, 0, s.stream>>>(s.g, d.lam, d.mu, d.vc, d.yy, d.mr, sta);
         s.launches++;
         SORD_CUDA(cudaGetLastError());
-        d.statics_made = true;
+        d.statics_there = d.statics_valid = true;
     }
     return sta;
 }

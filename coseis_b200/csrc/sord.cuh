@@ -216,8 +216,9 @@ struct Device {
     bool vol_plain = false;
     // k_modal's statics (per cell lam / V, mu / V, yy and a node's mr, 16
     // bytes) lie over sd[0..2] and so[0], which only the separate-kernel
-    // step uses: valid until that step runs or a modulus is set
-    bool statics_made = false;
+    // step uses and which that step clears first (statics_there); they hold
+    // until that step runs or a modulus is set (statics_valid)
+    bool statics_there = false, statics_valid = false;
 };
 
 // Fault-plane arrays (dynamic_rupture.f90:22-63), offsets into Device::fp.

@@ -1,0 +1,43 @@
+"""Steps of one kernel and steps of separate kernels on one handle, with the
+state written between them: what a step leaves in memory that the next one
+uses for something else must not show in its results."""
+import os
+
+import numpy as np
+import pytest
+
+import sordcases as sc
+
+
+@pytest.mark.gpu
+def test_moduli_set_before_a_separate_kernel_step(tmp_path, gpu_lib):
+    """Fast arithmetic, two steps of one kernel, moduli written back as they
+    were, then two steps that output the stress norm (separate kernels): all
+    bits as without the write.  The nodes on the faces read the stress of the
+    cells past the mesh, which is zero."""
+    from coseis_b200 import _lib
+    out = []
+    for write in (False, True):
+        d = str(tmp_path / str(write))
+        prm = {'shape': [21, 18, 16, 4], 'delta': [100.0, 100.0, 100.0, 0.0075], 'rho': [2670.0], 'vp': [6000.0],
+               'vs': [3464.0], 'gam': [0.1], 'hourglass': [1.0, 1.0], 'bc1': ['pml'] * 3, 'bc2': ['pml'] * 3,
+               'npml': 4, 'itstats': 1, 'itio': 4, 'mxy': [([10.5, 9.0, 8.0, []], '.', 1e14, 'ricker1', 0.02)],
+               'wm2': [([[], [], [], [2, None, 1]], '=>', 'wm2.bin')]}
+        sc.stage(prm, d)
+        s = _lib.Solver(d, open(os.path.join(d, 'sord.in')).read())
+        try:
+            s.set_arithmetic('fast')
+            s.step(2)
+            if write:
+                for f in ('lam', 'mu', 'yy'):
+                    s.set_field(f, s.field(f))
+            s.step(2)
+            v = [s.field('v' + a) for a in 'xyz']
+            stats = s.stats()
+        finally:
+            s.close()
+        out.append((np.fromfile(os.path.join(d, 'wm2.bin'), '<f4'), v, stats))
+    (w0, v0, s0), (w1, v1, s1) = out
+    assert np.abs(w0).max() > 0
+    assert np.array_equal(w0, w1) and s0 == s1, (s0, s1)
+    assert all(np.array_equal(a, b) for a, b in zip(v0, v1))
