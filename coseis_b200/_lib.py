@@ -156,8 +156,8 @@ def binomial_cost(nt, snapshots):
 
 
 def trim_memory(device=0):
-    """Wait for the device memory of destroyed handles to go back to the
-    driver (it is returned on a helper thread)."""
+    """Return the device memory of destroyed handles to the driver now (a
+    helper thread returns it, the last 2 GiB after ten seconds)."""
     _check(load().sord_trim_memory(device))
 
 

@@ -1,6 +1,10 @@
 // Device helpers used by setup, field I/O and statistics: fills, set_halo
 // (utilities.f90:103-117), region reductions, vector/tensor norms
 // (utilities.f90:120-165) and rinvert (utilities.f90:40-49).
+#include <unistd.h>
+
+#include <chrono>
+#include <condition_variable>
 #include <cstdint>
 #include <cstdlib>
 #include <map>
@@ -221,26 +225,55 @@ void smem_limit(const void* func, int bytes) {
 // neither grows the pool anew each time nor waits for the trim before it
 // (a gradient of 64^3 nodes and 120 kept states, 1.2 GiB: the forward run's
 // allocations 30 ms and the wait in sord_create 4 to 100 ms, now 9 ms for
-// the forward run and 2 ms to create; 1/90 of the device's memory is kept);
-// sord_trim_memory returns the rest.  Returning tens of GB to the driver
-// takes up to seconds, so the trim runs on a helper thread and the
-// destroying call returns at once; the next handle created on that device,
-// and the exit of the process (an atexit handler, registered after the CUDA
-// runtime's own and so run before it), wait for it.
+// the forward run and 2 ms to create; 1/90 of the device's memory is kept).
+// The rest goes back once no handle has been made for kPoolIdle, or at once
+// by sord_trim_memory.  Returning tens of GB to the driver takes up to
+// seconds, so both trims run on a helper thread and the destroying call
+// returns at once; the next handle created on that device, and the exit of
+// the process (an atexit handler, registered after the CUDA runtime's own
+// and so run before it), end its wait and wait for a trim under way.
 static constexpr uint64_t kPoolKeep = (uint64_t)2 << 30;
+static constexpr std::chrono::seconds kPoolIdle{10};
 static std::mutex g_mem_m;
-static std::map<int, int> g_live;             // device -> live handles
-static std::map<int, std::thread> g_trim;     // device -> trim in progress
+static std::map<int, int> g_live;  // device -> live handles
+struct Trim {
+    std::thread thread;
+    std::mutex m;
+    std::condition_variable cv;
+    bool stop = false;
+};
+static std::map<int, Trim> g_trim;  // device -> trim in progress
+static pid_t g_trim_pid = 0;        // process whose threads they are
+
+static void trim_end(Trim& t) {
+    if (!t.thread.joinable()) return;
+    if (g_trim_pid != getpid()) {  // in a forked child the thread is not there
+        t.thread.detach();
+        return;
+    }
+    {
+        std::lock_guard<std::mutex> lock(t.m);
+        t.stop = true;
+    }
+    t.cv.notify_all();
+    t.thread.join();
+}
 
 static void trim_join_locked(int device) {
     auto it = g_trim.find(device);
-    if (it != g_trim.end() && it->second.joinable()) it->second.join();
+    if (it != g_trim.end()) trim_end(it->second);
 }
 
 static void trim_join_all() {
     std::lock_guard<std::mutex> lock(g_mem_m);
-    for (auto& t : g_trim)
-        if (t.second.joinable()) t.second.join();
+    for (auto& t : g_trim) trim_end(t.second);
+}
+
+// Return the pool's unused memory, now and as it is freed.
+static cudaError_t pool_release(cudaMemPool_t pool) {
+    uint64_t none = 0;
+    const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &none);
+    return e != cudaSuccess ? e : cudaMemPoolTrimTo(pool, 0);
 }
 
 void mem_attach(int device) {
@@ -254,7 +287,7 @@ void mem_attach(int device) {
     }
 }
 
-// Wait for a pending trim on `device`; with no live handle there, return
+// End a pending trim on `device`; with no live handle there, return
 // the pool's unused memory to the driver now.
 void mem_trim(int device) {
     std::lock_guard<std::mutex> lock(g_mem_m);
@@ -262,7 +295,7 @@ void mem_trim(int device) {
     if (g_live[device] == 0) {
         cudaMemPool_t pool;
         SORD_CUDA(cudaDeviceGetDefaultMemPool(&pool, device));
-        SORD_CUDA(cudaMemPoolTrimTo(pool, 0));
+        SORD_CUDA(pool_release(pool));
     }
 }
 
@@ -272,15 +305,23 @@ void mem_detach(int device) {
     if (--g_live[device] == 0) {
         cudaMemPool_t pool;
         if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
-            uint64_t keep = kPoolKeep, held = ~0ull;
+            uint64_t keep = kPoolKeep;
             cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
             trim_join_locked(device);
-            if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess && held <= keep) return;
             std::call_once(at_exit, [] { std::atexit(trim_join_all); });
-            g_trim[device] = std::thread([device, pool] {
-                cudaSetDevice(device);
-                cudaMemPoolTrimTo(pool, kPoolKeep);
-            });
+            Trim& t = g_trim[device];
+            t.stop = false;
+            try {
+                t.thread = std::thread([device, pool, &t] {
+                    cudaSetDevice(device);
+                    cudaMemPoolTrimTo(pool, kPoolKeep);
+                    std::unique_lock<std::mutex> lock(t.m);
+                    if (!t.cv.wait_for(lock, kPoolIdle, [&t] { return t.stop; })) pool_release(pool);
+                });
+                g_trim_pid = getpid();
+            } catch (const std::exception&) {  // no thread to be had
+                pool_release(pool);
+            }
         }
     }
 }

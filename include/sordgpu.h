@@ -151,12 +151,12 @@ int sord_adjoint_backward(sord_handle* h, int nrec, const char* const* files, co
 
 /* Device memory of the handles comes from the device's default memory
  * pool; when the last handle on a device is destroyed the pool's memory is
- * returned to the driver, all but 2 GiB that the next handle may use, on
- * a helper thread, so sord_destroy and sord_run_directory return without
- * waiting for it.  sord_trim_memory
- * waits for that, and with no live handle on `device` returns the pool's
- * unused memory now: call it before allocating the memory elsewhere in the
- * same process.  No reference counterpart (the reference frees its arrays
+ * returned to the driver on a helper thread, so sord_destroy and
+ * sord_run_directory return without waiting for it: all but 2 GiB, which the
+ * next handle may use, at once, and those when ten seconds have passed
+ * without one.  sord_trim_memory with no live handle on `device` returns
+ * the pool's unused memory now: call it before allocating the memory
+ * elsewhere.  No reference counterpart (the reference frees its arrays
  * at process exit). */
 int sord_trim_memory(int device);
 
