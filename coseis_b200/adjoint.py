@@ -125,7 +125,8 @@ def material_chain(rho, vp, vs, g, delta):
     Arrays are indexed [j, k, l]; computed in float64.  ReceiverTraces has
     the library do this on the device (Solver.adjoint_material: 28 ms here for
     63^3 cells, 60 passes over arrays that numpy allocates anew), in the same
-    order of operations."""
+    order of operations, and falls back to this where the device memory that
+    takes (48 bytes per cell, about 200 MB at most) is not to be had."""
     rho = np.asarray(rho, np.float64)
     vp = np.asarray(vp, np.float64)
     vs = np.asarray(vs, np.float64)
@@ -209,8 +210,14 @@ def _function():
             dtr = {f: g[i // 3, i % 3] for i, f in enumerate(files)}
             try:
                 res = ctx.solver.adjoint_backward(dtr, len(ctx.order))
-                grho, gvp, gvs = ctx.solver.adjoint_material(rho.detach().cpu().numpy(), vp.detach().cpu().numpy(),
-                                                             vs.detach().cpu().numpy(), p.prm['delta'])
+                vals = [a.detach().cpu().numpy() for a in (rho, vp, vs)]
+                try:
+                    grho, gvp, gvs = ctx.solver.adjoint_material(*vals, p.prm['delta'])
+                except _lib.SordError as e:
+                    # the kept states may leave no room for its device scratch
+                    if e.code != _lib.SORD_E_NOMEM:
+                        raise
+                    grho, gvp, gvs = material_chain(*vals, res, p.prm['delta'])
             finally:
                 ctx.solver.close()
                 shutil.rmtree(ctx.dir, ignore_errors=True)
