@@ -1060,6 +1060,7 @@ static void field_io_op(Solver& s, size_t opi, FieldView f, OutBatch& out) {
 static void finish_outputs(Solver& s, OutBatch& batch) {
     launch_outputs(s, batch);
     for (OutBatch::Full& f : batch.full) flush_output(s, s.ops[f.op], f.n, f.m);
+    batch.full.clear();
 }
 
 // One pass of a field's hooks; outputs are left in `batch`.
@@ -1068,7 +1069,9 @@ static void field_io_pass(Solver& s, char pass, const char* field, FieldView f, 
     for (size_t i = 0; i < s.ops.size(); i++) {
         if (applies(s, s.ops[i], field, pass, true)) any = true;
         if (!applies(s, s.ops[i], field, pass)) continue;
-        if (pass == '<') launch_outputs(s, batch);  // what they read is still as it was
+        // what the outputs so far read is still as it was, and they are
+        // written whether or not this input can be read
+        if (pass == '<') finish_outputs(s, batch);
         field_io_op(s, i, f, batch);
     }
     // a partitioned run takes the halo planes of an input volume field
