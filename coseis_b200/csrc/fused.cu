@@ -1098,6 +1098,16 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
 #include "shell.cuh"
 #include "slab.cuh"
 
+// Arithmetic of the fused step.  The fast PML kernels give a cell or node one
+// memory per axis, so a mesh on which the bands of opposite faces share cells
+// (the front end refuses it, a deck need not) takes the kernels in reference
+// order, which apply both, the near one first, as the reference does.
+static int step_arith(const Solver& s) {
+    for (int d = 0; d < 3; d++)
+        if (s.g.npml > 0 && s.g.i2pml[d] - 1 <= s.g.i1pml[d]) return 0;
+    return s.arith;
+}
+
 // Work decomposition of a fused step, fixed by the mesh.  The interior
 // rectangle holds the node columns (j, k) whose adjacent cells all lie
 // strictly inside the non-PML region, jf..jend x kf..kend; it is tiled by
@@ -1175,7 +1185,7 @@ static void push_box(std::vector<int>& v, int ipl, int j1, int j2, int k1, int k
 }
 
 static FusedPlan& fused_plan(Solver& s) {
-    if (s.fplan && s.fplan->arith == s.arith) return *s.fplan;
+    if (s.fplan && s.fplan->arith == step_arith(s)) return *s.fplan;
     if (s.fplan) {
         // the arithmetic was changed between two steps
         SORD_CUDA(cudaStreamSynchronize(s.stream));
@@ -1183,7 +1193,7 @@ static FusedPlan& fused_plan(Solver& s) {
     }
     FusedPlan* P = new FusedPlan();
     s.fplan = P;
-    P->arith = s.arith;
+    P->arith = step_arith(s);
     // shortest plane range of a launch that does not fill the chip
     const int few = kFewPlanes;
     const Geom& g = s.g;
@@ -1268,7 +1278,7 @@ static FusedPlan& fused_plan(Solver& s) {
         };
         int ipl = kItemPlanes;
         while (ipl > kMinPlanes && count(ipl) < want) ipl = std::max(kMinPlanes, ipl * 2 / 3);
-        while (ipl > few && count(ipl) < (s.arith ? sms : 2 * sms)) ipl = std::max(few, ipl * 2 / 3);
+        while (ipl > few && count(ipl) < (step_arith(s) ? sms : 2 * sms)) ipl = std::max(few, ipl * 2 / 3);
         iplc[c] = ipl;
     }
     // boxes by their own class (a range of planes may miss the PML of z)
@@ -1343,7 +1353,7 @@ static void launch_modal(Solver& s, const StepArgs& A, dim3 grid, cudaStream_t s
 // whose cells are not boxes (a constant shear) takes the general kernels,
 // since k_modal has the axes' own modes only.
 static int step_class(const Solver& s) {
-    if (!s.arith) return s.geom;
+    if (!step_arith(s)) return s.geom;
     // k_modal damps every node by dt hg2 in the PML; the reference leaves it
     // out there for a negative constant
     if (s.prm.hourglass[1] < 0.f) return GEOM_GENERAL;
@@ -1368,13 +1378,13 @@ template <int GEOM>
 static void launch_interior(Solver& s, const StepArgs& A, dim3 grid, cudaStream_t st) {
     constexpr bool FM = GEOM == GEOM_GENERAL;  // fast arithmetic of the other meshes: k_modal
     if constexpr (!FM) {
-        if (s.arith) {
+        if (step_arith(s)) {
             launch_modal<GEOM, 0>(s, A, grid, st);
             return;
         }
     }
-    const size_t bytes = FM && s.arith ? Lay<GEOM>::bytes_fm : Lay<GEOM>::bytes;
-    auto kern = FM && s.arith ? k_interior<GEOM, FM> : k_interior<GEOM, false>;
+    const size_t bytes = FM && step_arith(s) ? Lay<GEOM>::bytes_fm : Lay<GEOM>::bytes;
+    auto kern = FM && step_arith(s) ? k_interior<GEOM, FM> : k_interior<GEOM, false>;
     smem_limit((const void*)kern, (int)bytes);
     kern<<<grid, dim3(FJ, FK), bytes, st>>>(A);
     s.launches++;
@@ -1384,7 +1394,7 @@ static void launch_interior(Solver& s, const StepArgs& A, dim3 grid, cudaStream_
 // Boxes of the PML shell of one class.
 template <int GEOM, int MASK>
 static void launch_boxes(Solver& s, const StepArgs& A, unsigned n, cudaStream_t st) {
-    if (s.arith) {
+    if (step_arith(s)) {
         if constexpr (GEOM != GEOM_GENERAL) {
             launch_modal<GEOM, MASK>(s, A, dim3(n, 1, 1), st);
             return;
@@ -1489,7 +1499,7 @@ void launch_fused(Solver& s, const InjectList& pot, const InjectList& mom, const
     for (int d = 0; d < 6; d++) A.ibox[d] = ib[d];
 
     const int geom = step_class(s);
-    A.sta = s.arith && geom != GEOM_GENERAL ? modal_statics(s) : nullptr;
+    A.sta = step_arith(s) && geom != GEOM_GENERAL ? modal_statics(s) : nullptr;
 
     cudaEvent_t e0 = nullptr;
     s.prof_begin(KC_FUSED, &e0);

@@ -219,9 +219,10 @@ double sord_last_step_ms(const sord_handle* h);
  * support-operator brackets scaled by h once per cell, each divergence
  * bracket taken as the negated gradient bracket of the same cell and corner;
  * equal to mode 0 in exact arithmetic, FP32 rounding apart.  The fault
- * kernels and the steps that run as separate kernels keep mode 0.  New handles start in mode 1 when the
- * environment variable SORD_ARITHMETIC is "fast".  May be called between any
- * two steps.  sord_get_arithmetic returns the mode. */
+ * kernels, the steps that run as separate kernels and meshes on which the
+ * PML bands of opposite faces share cells keep mode 0.  New handles start in
+ * mode 1 when the environment variable SORD_ARITHMETIC is "fast".  May be
+ * called between any two steps.  sord_get_arithmetic returns the mode. */
 int sord_set_arithmetic(sord_handle* h, int mode);
 int sord_get_arithmetic(const sord_handle* h);
 
