@@ -1118,7 +1118,7 @@ static int step_arith(const Solver& s) {
 // covered by masked 15 x 15 node boxes for the shell kernel.  Boxes and tiles partition
 // the nodes, so every node, and every PML memory, is updated once.
 struct FusedPlan {
-    int arith = 0;                              // the arithmetic it was made for
+    bool ready = false;                         // all of it is there
     int jf = 0, jend = -1, kf = 0, kend = -1;   // interior rectangle (inclusive)
     int nbx = 0, nby = 0;                       // interior tiles
     int lf0 = 0, lf1 = -1;                      // interior node planes (inclusive)
@@ -1137,8 +1137,7 @@ struct FusedPlan {
     cudaEvent_t cfork = nullptr, cdone[4] = {};
 };
 
-void fused_free(Solver& s) {
-    FusedPlan* P = s.fplan;
+static void plan_free(Solver& s, FusedPlan*& P) {
     if (!P) return;
     if (P->fork) cudaEventDestroy(P->fork);
     if (P->join) cudaEventDestroy(P->join);
@@ -1150,7 +1149,10 @@ void fused_free(Solver& s) {
     }
     dev_free(s, P->d_items);
     delete P;
-    s.fplan = nullptr;
+    P = nullptr;
+}
+void fused_free(Solver& s) {
+    for (FusedPlan*& P : s.fplan) plan_free(s, P);
 }
 
 // Planes per block.  Each block streams its column through the planes, so
@@ -1185,15 +1187,11 @@ static void push_box(std::vector<int>& v, int ipl, int j1, int j2, int k1, int k
 }
 
 static FusedPlan& fused_plan(Solver& s) {
-    if (s.fplan && s.fplan->arith == step_arith(s)) return *s.fplan;
-    if (s.fplan) {
-        // the arithmetic was changed between two steps
-        SORD_CUDA(cudaStreamSynchronize(s.stream));
-        fused_free(s);
-    }
-    FusedPlan* P = new FusedPlan();
-    s.fplan = P;
-    P->arith = step_arith(s);
+    // one for each arithmetic, which may change between any two steps
+    FusedPlan*& P = s.fplan[step_arith(s)];
+    if (P && P->ready) return *P;
+    plan_free(s, P);
+    P = new FusedPlan();
     // shortest plane range of a launch that does not fill the chip
     const int few = kFewPlanes;
     const Geom& g = s.g;
@@ -1332,6 +1330,7 @@ static FusedPlan& fused_plan(Solver& s) {
         SORD_CUDA(cudaEventCreateWithFlags(&P->cdone[c], cudaEventDisableTiming));
         SORD_CUDA(cudaStreamCreateWithFlags(&P->cst[c], cudaStreamNonBlocking));
     }
+    P->ready = true;
     return *P;
 }
 

@@ -348,7 +348,7 @@ struct Solver {
     cudaEvent_t pin_ev[8] = {};
     int rec_slot = 0;          // next chunk buffer for a time-varying input record
     // work decomposition of the fused step kernels (fused.cu)
-    FusedPlan* fplan = nullptr;
+    FusedPlan* fplan[2] = {};  // by arithmetic
     struct AdjointState* adj = nullptr;  // checkpoints and adjoint fields (adjoint.cu)
     struct OutWriter* writer = nullptr;  // output-record writer thread (fieldio.cu)
     // partitioned run (sord_create_part): part `part` of `nparts` slabs along

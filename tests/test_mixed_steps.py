@@ -41,3 +41,36 @@ def test_moduli_set_before_a_separate_kernel_step(tmp_path, gpu_lib):
     assert np.abs(w0).max() > 0
     assert np.array_equal(w0, w1) and s0 == s1, (s0, s1)
     assert all(np.array_equal(a, b) for a, b in zip(v0, v1))
+
+
+@pytest.mark.gpu
+def test_arithmetic_changed_at_every_step(tmp_path, gpu_lib):
+    """sord_set_arithmetic may be called between any two steps: a step after
+    a change takes no more than three times the slower of the two
+    arithmetics, and the state stays that of the reference to 1e-5."""
+    import time
+    from coseis_b200 import _lib
+    took, out = {}, {}
+    for name, modes in (('reference', ['reference']), ('fast', ['fast']), ('both', ['reference', 'fast'])):
+        d = str(tmp_path / name)
+        prm = {'shape': [96, 80, 72, 10 ** 6], 'delta': [100.0, 100.0, 100.0, 0.008], 'rho': [2670.0],
+               'vp': [6000.0], 'vs': [3464.0], 'gam': [0.1], 'hourglass': [1.0, 1.0], 'bc1': ['pml'] * 3,
+               'bc2': ['pml'] * 3, 'npml': 10, 'itstats': 10 ** 6, 'itio': 10 ** 6,
+               'mxy': [([48.5, 40.0, 36.0, []], '.', 1e14, 'ricker1', 0.02)]}
+        sc.stage(prm, d)
+        s = _lib.Solver(d, open(os.path.join(d, 'sord.in')).read())
+        try:
+            best = float('inf')
+            for rep in range(4):
+                t = time.perf_counter()
+                for i in range(40):
+                    s.set_arithmetic(modes[i % len(modes)])
+                    s.step(1)
+                best = min(best, time.perf_counter() - t)
+            took[name] = best
+            out[name] = np.concatenate([s.field('v' + a).ravel() for a in 'xyz']).astype(float)
+        finally:
+            s.close()
+    n = np.linalg.norm(out['reference'])
+    assert n > 0 and all(np.linalg.norm(v - out['reference']) <= 1e-5 * n for v in out.values())
+    assert took['both'] <= 3 * max(took['reference'], took['fast']), took
