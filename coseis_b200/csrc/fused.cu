@@ -10,21 +10,21 @@
 //                a = f * mr, and the leapfrog update of the NEXT step
 //                v' = v + dt a, u' = u + dt v' (time_integration.f90:27-41)
 //
-// Each block owns a 31 x 7 column of output nodes (32 x 8 cells including
-// the -1 halo) and streams along l.  Node planes are staged raw (u, v, gam,
-// coordinates) by cp.async into shared memory one plane ahead, then turned
-// into a 3-plane ring of the per-node values the cells need: w = u + gam v,
-// the hourglass input hg1 u + dt hg2 v, and the coordinates.  Cell planes
-// (stress, hourglass values, divergence brackets) sit in a 2-plane ring.
-// Two barriers per plane.  Cells on tile borders are computed by both
-// neighbours (from identical inputs, so identically); the owner writes the
-// PML g memory, which is double-buffered like v and u so no block reads a
-// value another block has already advanced.
+// A block of the interior kernel owns a 31 x 7 column of output nodes (32 x 8
+// cells including the -1 halo) and streams along l.  Node planes are staged
+// raw (u, v, gam, coordinates) by cp.async into shared memory one plane ahead,
+// then turned into a 3-plane ring of the per-node values the cells need:
+// w = u + gam v, the hourglass input hg1 u + dt hg2 v, and the coordinates.
+// Cell planes (stress, hourglass values, divergence brackets) sit in a 2-plane
+// ring.  Two barriers per plane.  Cells on tile borders are computed by both
+// neighbours (from identical inputs, so identically).
 //
-// Planes of blocks whose whole tile lies outside the PML, with no point
-// source in the block, run a fast path with the PML, boundary and injection
-// branches compiled out; the arithmetic of both paths is the same, so a
-// cell computed by either is bit-identical.
+// Nodes with a PML cell or node around them are left to the shell's kernels
+// (shell.cuh; fast arithmetic on general meshes: slab.cuh), on the same plan:
+// the owner of a cell writes its PML g memory, which is double-buffered like
+// v and u so no block reads a value another block has already advanced.  In
+// reference order the operations of a cell are the same in both, so a cell
+// computed by either is bit-identical.  Point sources are applied in all.
 //
 // Support-operator brackets: rectilinear meshes use the per-direction
 // constants verified at setup; terrain meshes (x = x(j), y = y(k)) compute
@@ -39,7 +39,6 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
-#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -86,15 +85,9 @@ struct Lay {
     static constexpr int NGC = GEOM == GEOM_RECT ? 5 : GEOM == GEOM_TERRAIN ? 9 : 11;  // float4 groups per cell
     static constexpr size_t bytes = sizeof(float) * (size_t)RAWSZ + sizeof(float4) * (size_t)(3 * NPL * NGN + 2 * NCL * NGC);
     // fast arithmetic: one cell plane (each node plane reads only the cells
-    // above it); groups: (e11 e22 e33 e23), (e31 e12) as float2, then per
-    // reading node column q: its hourglass sums for the node above and
-    // below, and its divergence brackets (NQ groups)
-    // (terrain: 2 groups per q, the lower-cell brackets of all q in 2 float2 groups)
-    static constexpr int NQ = NDIR == 3 ? 3 : 2;
-    static constexpr int NGCF = 2 + 4 * NQ + (NDIR == 2 ? 2 : 0);
-    // the interior kernel in fast arithmetic stores, per reading node column
-    // q, that node's whole force terms from the cell: (fu_x, fu_y, fu_z,
-    // fl_x) as float4 group q and (fl_y, fl_z) as float2 in groups 4-5
+    // above it), which holds, per reading node column q, that node's whole
+    // force terms from the cell: (fu_x, fu_y, fu_z, fl_x) as float4 group q
+    // and (fl_y, fl_z) as float2 in groups 4-5
     static constexpr int NGCR = 6;
     static constexpr size_t bytes_fm = sizeof(float) * (size_t)RAWSZ + sizeof(float4) * (size_t)(3 * NPL * NGN + NCL * NGCR);
 };
@@ -182,24 +175,16 @@ __device__ __forceinline__ long long slab_idx(const Geom& g, int axis, int t, in
 
 constexpr int SJ = 16, SK = 16;  // shell tile (cells = threads)
 
-// Zero one cell of the fast-arithmetic cell plane (layout of Lay: NGCF
-// groups of ncl float4) in the pattern the cell phase writes it: group 1
-// and, with two bracket directions, the lower-bracket groups hold float2
-// values at index tid, which a float4 store at tid would miss (and would
-// clear two other cells' values instead).
-template <int NDIR, int NQ>
+// Zero one cell of the fast-arithmetic cell plane of the shell (layout of
+// LaySl: NGCF groups of ncl float4) in the pattern the cell phase writes it:
+// group 1 holds float2 values at index tid, which a float4 store at tid would
+// miss (and would clear two other cells' values instead).
 __device__ __forceinline__ void zero_cell_fm(float4* sC, int tid, int ncl) {
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
     sC[tid] = z;
     reinterpret_cast<float2*>(sC + ncl)[tid] = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        float4* cq = sC + (2 + NQ * q) * ncl + tid;
-        cq[0] = z;
-        cq[ncl] = z;
-        if (NDIR == 3) cq[2 * ncl] = z;
-        if (NDIR == 2) reinterpret_cast<float2*>(sC + (2 + 4 * NQ) * ncl)[q * ncl + tid] = make_float2(0.f, 0.f);
-    }
+    for (int i = 2; i < 14; i++) sC[i * ncl + tid] = z;
 }
 
 // Zero one cell of the interior kernel's fast-arithmetic cell plane (Lay:
@@ -372,11 +357,9 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
     // fast arithmetic: the terms of this thread's own cell for its own node
     // column (reader q = 0) stay in registers for the node phase
     float ownu[3] = {0.f, 0.f, 0.f}, ownl[3] = {0.f, 0.f, 0.f};
-    auto cells = [&](int l, auto fast_tag) {
-        constexpr bool F = decltype(fast_tag)::value;
+    auto cells = [&](int l) {
         const int cs = FM ? 0 : l & 1;
-        const bool valid = (F || cellcol) && l >= g.i1cell[2] && l <= g.i2cell[2];
-        if (!valid) {
+        if (!(l >= g.i1cell[2] && l <= g.i2cell[2])) {
             if constexpr (FM) {
                 zero_cell_fr(sC, tid, NCL);
 #pragma unroll
@@ -472,7 +455,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
 #pragma unroll
         for (int i = 0; i < 12; i++) he[i] = 0.f;
         const bool own = owncol && l >= L0;
-        if constexpr (F && FM) {
+        if constexpr (FM) {
             // gradients; the off-diagonal pairs are summed here and halved
             // with the modulus below
             float sg[3][3];
@@ -489,7 +472,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
             eo[0] = sg[1][2] + sg[2][1];
             eo[1] = sg[0][2] + sg[2][0];
             eo[2] = sg[0][1] + sg[1][0];
-        } else if constexpr (F && !kPaired) {
+        } else if constexpr (!kPaired) {
 #pragma unroll
             for (int ic = 0; ic < 3; ic++) {
                 float W[8];
@@ -504,7 +487,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
                     else eo[3 - ic - id] = eo[3 - ic - id] + 0.5f * s;
                 }
             }
-        } else if constexpr (F) {
+        } else {
             // strain of an interior cell: s[ic][id] = stencil8(w_ic, B[id]);
             // (ic0, ic1) paired per iid, ic2's first two directions paired
             const F2 h2 = f2(h, nz);
@@ -544,83 +527,6 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
             eo[0] = 0.5f * sg[1][2] + 0.5f * sg[2][1];
             eo[1] = 0.5f * sg[0][2] + 0.5f * sg[2][0];
             eo[2] = 0.5f * sg[0][1] + 0.5f * sg[1][0];
-        } else {
-            // region of the cell (stress.f90:141-248)
-            bool nearS[3], farS[3], anyS = false;
-            const int cc[3] = {J, K, l};
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                nearS[d] = cc[d] <= g.i1pml[d];
-                farS[d] = cc[d] >= g.i2pml[d] - 1;
-                anyS = anyS || nearS[d] || farS[d];
-            }
-            // PML cells that are not elastic-hourglass cells carry the viscous
-            // hourglass values dt hg2 yy hourglass_nc(v) in the hourglass
-            // slots (acceleration.f90:164-183)
-            bool inEc = true;
-#pragma unroll
-            for (int d = 0; d < 3; d++) inEc = inEc && cc[d] >= g.i1pml[d] && cc[d] <= g.i2pml[d] - 1;
-            const bool visc = A.hourglass && A.hgvisc && anyS && !inEc;
-            const float yv = A.dh2 * cur[3];
-#pragma unroll
-            for (int i = 0; i < 3; i++) { ed[i] = 0.f; eo[i] = 0.f; }
-#pragma unroll
-            for (int ic = 0; ic < 3; ic++) {
-                float W[8], U[8], V[8];
-#pragma unroll
-                for (int t = 0; t < 8; t++) {
-                    W[t] = Wc[ic][term_corner(t)];
-                    U[t] = 0.f;
-                    V[t] = 0.f;
-                }
-                if (anyS) {
-#pragma unroll
-                    for (int t = 0; t < 8; t++) {
-                        const int n = term_corner(t);
-                        const long long qn = g.idx(J + (n & 1), K + ((n >> 1) & 1), l + (n >> 2));
-                        U[t] = A.uin[ic][qn];
-                        V[t] = A.vin[ic][qn];
-                    }
-                }
-                if (visc) {
-                    float Vc[8], Vh[8];
-#pragma unroll
-                    for (int t = 0; t < 8; t++) Vc[term_corner(t)] = V[t];
-#pragma unroll
-                    for (int t = 0; t < 8; t++) Vh[t] = Vc[hg_corner(t)];
-#pragma unroll
-                    for (int iq = 0; iq < 4; iq++) he[3 * iq + ic] = yv * hg_sum(Vh, iq);
-                }
-#pragma unroll
-                for (int iid = 0; iid < 3; iid++) {
-                    const int id = (ic + iid + 1) % 3;
-                    float s;
-                    if (nearS[id] || farS[id]) {
-                        const float raw = stencil8(V, B[id], h);
-                        s = raw;
-                        const int c = cc[id];
-                        if (nearS[id]) {
-                            const int p = c + g.nnoff[id];
-                            const long long gi = slab_idx(g, id, A.sl.tg[id], c - g.i1cell[id], J, K, l, ic);
-                            s = A.pmlc[3 * g.npml + p - 1] * raw + A.pmlc[2 * g.npml + p - 1] * A.sl.g[id][gi];
-                            if (own) A.gout[id][gi] = s;
-                        }
-                        if (farS[id]) {
-                            const int p = g.nn[id] - c - g.nnoff[id];
-                            const long long gi = slab_idx(g, id, A.sl.tg[3 + id], g.i2cell[id] - c, J, K, l, ic);
-                            s = A.pmlc[3 * g.npml + p - 1] * raw + A.pmlc[2 * g.npml + p - 1] * A.sl.g[3 + id][gi];
-                            if (own) A.gout[3 + id][gi] = s;
-                        }
-                    } else if (anyS) {
-                        s = stencil8(U, B[id], h);
-                    } else {
-                        s = stencil8(W, B[id], h);
-                    }
-                    if (ic == id) ed[ic] = s;
-                    else if (ic < id) eo[3 - ic - id] = 0.5f * s;
-                    else eo[3 - ic - id] = eo[3 - ic - id] + 0.5f * s;
-                }
-            }
         }
         const bool src = scol && l >= A.ibox[2] && l <= A.ibox[5];
         if (src && npot != 0) {
@@ -661,13 +567,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
             st_w = fmaxn(st_w, (ed[0] * ed[0] + ed[1] * ed[1] + ed[2] * ed[2]) + 2.0f * (eo[0] * eo[0] + eo[1] * eo[1] + eo[2] * eo[2]));
         // elastic hourglass cell values (acceleration.f90:141-156)
         if (A.hourglass) {
-            bool inE = true;
-            if constexpr (!F) {
-                const int cc[3] = {J, K, l};
-#pragma unroll
-                for (int d = 0; d < 3; d++) inE = inE && cc[d] >= g.i1pml[d] && cc[d] <= g.i2pml[d] - 1;
-            }
-            if (FM && inE) {
+            if constexpr (FM) {
                 // the four mode sums by butterflies (stencil.cuh: hg_modes)
                 const float y = cur[3];
 #pragma unroll
@@ -677,7 +577,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
 #pragma unroll
                     for (int iq = 0; iq < 4; iq++) he[3 * iq + ic] = m[iq] * y;
                 }
-            } else if (inE && (!F || !kPaired)) {
+            } else if constexpr (!kPaired) {
                 const float y = cur[3];
 #pragma unroll
                 for (int ic = 0; ic < 3; ic++) {
@@ -687,7 +587,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
 #pragma unroll
                     for (int iq = 0; iq < 4; iq++) he[3 * iq + ic] = hg_sum(W2, iq) * y;
                 }
-            } else if (inE) {
+            } else {
                 const float y = cur[3];
                 F2 H01[8];
                 float H2v[8];
@@ -725,12 +625,6 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
             for (int q = 0; q < 4; q++) {
                 const int cj = q & 1, ck = q >> 1;
                 const int tu = cj + 2 + 4 * ck, tl = cj + 4 * ck;
-                float Bu[3], Bl[3];
-#pragma unroll
-                for (int a = 0; a < 3; a++) {
-                    Bu[a] = a < NDIR ? cnb[a < NDIR ? a : 0][tu] : A.brh.bcn[a][tu];
-                    Bl[a] = a < NDIR ? cnb[a < NDIR ? a : 0][tl] : A.brh.bcn[a][tl];
-                }
                 float fu[3], fl[3];
 #pragma unroll
                 for (int ic = 0; ic < 3; ic++) hg_reader<float>(hr[ic], q, fu[ic], fl[ic]);
@@ -739,8 +633,8 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
 #pragma unroll
                     for (int iid = 0; iid < 3; iid++) {
                         const int id = (ic + iid) % 3, comp = ic == id ? ic : 3 + (3 - ic - id);
-                        fu[ic] = fmaf(S[comp], Bu[id], fu[ic]);
-                        fl[ic] = fmaf(S[comp], Bl[id], fl[ic]);
+                        fu[ic] = fmaf(S[comp], cnb[id][tu], fu[ic]);
+                        fl[ic] = fmaf(S[comp], cnb[id][tl], fl[ic]);
                     }
                 if (q == 0) {
 #pragma unroll
@@ -775,8 +669,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
     // at (J + cj, K + ck, l - 1 + cl); diff_cn term t sits at position
     // pt(t), hourglass_cn term t at position ph(t).
     // (reference order only; fast arithmetic uses nodes_fm below)
-    auto nodes = [&](int l, auto fast_tag) {
-        constexpr bool F = decltype(fast_tag)::value;
+    auto nodes = [&](int l) {
         if (!outcol) return;
         const long long q = g.idx(jn, kn, l);
         const float4* c0 = sC + ((l - 1) & 1) * (NGC * NCL) + tid;  // cell plane l-1
@@ -808,7 +701,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
             if (GEOM == GEOM_TERRAIN) Bc[2][t] = A.br.bcn[2][t];
         }
         float f[3];
-        if constexpr (F && !kPaired) {
+        if constexpr (!kPaired) {
 #pragma unroll
             for (int ic = 0; ic < 3; ic++)
 #pragma unroll
@@ -818,7 +711,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
                     const float s = stencil8(S[comp], Bc[id], h);
                     f[ic] = iid == 0 ? s : f[ic] + s;
                 }
-        } else if constexpr (F) {
+        } else {
             // f[ic] = sum over iid of stencil8(sigma(ic, id), Bc[id]), id = (ic + iid) % 3;
             // (ic0, ic1) paired per iid, ic2's first two terms paired
             const F2 h2 = f2(h, nz);
@@ -847,38 +740,8 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
             f[2] = f[2] + stencil8<float>(S[3], Bc[1], h);
             f[0] = f01.x();
             f[1] = f01.y();
-        } else {
-#pragma unroll
-            for (int ic = 0; ic < 3; ic++) {
-#pragma unroll
-                for (int iid = 0; iid < 3; iid++) {
-                    const int id = (ic + iid) % 3;
-                    const int comp = ic == id ? ic : 3 + (3 - ic - id);
-                    float s = stencil8(S[comp], Bc[id], h);
-                    const int c = id == 0 ? jn : id == 1 ? kn : l;
-                    if (c <= g.i1pml[id]) {
-                        const int p = c + g.nnoff[id];
-                        float* P = A.sl.p[id] + slab_idx(g, id, A.sl.tp[id], c - g.i1node[id], jn, kn, l, ic);
-                        s = A.pmlc[g.npml + p - 1] * s + A.pmlc[p - 1] * *P;
-                        *P = *P + dt * s;
-                    }
-                    if (c >= g.i2pml[id]) {
-                        const int p = g.nn[id] - c - g.nnoff[id] + 1;
-                        float* P = A.sl.p[3 + id] + slab_idx(g, id, A.sl.tp[3 + id], g.i2node[id] - c, jn, kn, l, ic);
-                        s = A.pmlc[g.npml + p - 1] * s + A.pmlc[p - 1] * *P;
-                        *P = *P + dt * s;
-                    }
-                    f[ic] = iid == 0 ? s : f[ic] + s;
-                }
-            }
         }
         if (A.hourglass) {
-            bool ne = true;
-            if constexpr (!F) {
-                const int cn_[3] = {jn, kn, l};
-#pragma unroll
-                for (int d = 0; d < 3; d++) ne = ne && cn_[d] >= g.i1pml[d] + 1 && cn_[d] <= g.i2pml[d] - 1;
-            }
             // hourglass values of mode iq by hourglass_cn term: (x, y) pair and z
 #define HVALS(iq, hA, hB)                                                      \
     _Pragma("unroll") for (int t = 0; t < 8; t++) {                            \
@@ -901,7 +764,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
             hB[t] = cp_[4 * NCL].y;                                            \
         }                                                                      \
     }
-            if (ne && F && !kPaired) {
+            if constexpr (!kPaired) {
                 // each cell's hourglass groups once, as 128 / 64-bit loads:
                 // g1.zw = mode 0 (x, y), g2 = modes 1, 2 (x, y), g3 = mode 3
                 // (x, y), z of modes 0, 1, g4 = z of modes 2, 3
@@ -923,20 +786,7 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
                 for (int iq = 0; iq < 4; iq++)
 #pragma unroll
                     for (int ic = 0; ic < 3; ic++) f[ic] = f[ic] - hg_sum(H[iq][ic], iq);
-            } else if (ne && (!F || !kPaired)) {
-#pragma unroll
-                for (int iq = 0; iq < 4; iq++) {
-                    F2 hA[8];
-                    float hB[8];
-                    HVALS(iq, hA, hB);
-                    float Hx[8], Hy[8];
-#pragma unroll
-                    for (int t = 0; t < 8; t++) { Hx[t] = hA[t].x(); Hy[t] = hA[t].y(); }
-                    f[0] = f[0] - hg_sum(Hx, iq);
-                    f[1] = f[1] - hg_sum(Hy, iq);
-                    f[2] = f[2] - hg_sum(hB, iq);
-                }
-            } else if (ne) {
+            } else {
                 F2 f01 = f2(f[0], f[1], nz);
 #pragma unroll
                 for (int iq = 0; iq < 4; iq++) {
@@ -948,66 +798,6 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
                 }
                 f[0] = f01.x();
                 f[1] = f01.y();
-            } else if constexpr (!F) {
-                if (A.hgvisc) {
-                    // viscous-only hourglass in the PML (acceleration.f90:164-199):
-                    // every cell of a PML node is a PML cell; pure PML cells
-                    // hold their viscous values in the hourglass slots, cells
-                    // that are also elastic-hourglass cells (the layer next to
-                    // the elastic region) are evaluated here from v
-                    int kind[8];
-                    float yc[8];
-#pragma unroll
-                    for (int t = 0; t < 8; t++) {
-                        const int o = hg_corner(t);
-                        const int Jc = jn - (o & 1), Kc = kn - ((o >> 1) & 1), Lc = l - (o >> 2);
-                        const bool real = Jc >= g.i1cell[0] && Jc <= g.i2cell[0] && Kc >= g.i1cell[1] &&
-                                          Kc <= g.i2cell[1] && Lc >= g.i1cell[2] && Lc <= g.i2cell[2];
-                        const bool slab = Jc <= g.i1pml[0] || Jc >= g.i2pml[0] - 1 || Kc <= g.i1pml[1] ||
-                                          Kc >= g.i2pml[1] - 1 || Lc <= g.i1pml[2] || Lc >= g.i2pml[2] - 1;
-                        const bool inEc = Jc >= g.i1pml[0] && Jc <= g.i2pml[0] - 1 && Kc >= g.i1pml[1] &&
-                                          Kc <= g.i2pml[1] - 1 && Lc >= g.i1pml[2] && Lc <= g.i2pml[2] - 1;
-                        kind[t] = !(real && slab) ? 0 : inEc ? 2 : 1;
-                        yc[t] = kind[t] == 2 ? A.dh2 * A.yy[g.idx(Jc, Kc, Lc)] : 0.f;
-                    }
-#pragma unroll
-                    for (int iq = 0; iq < 4; iq++) {
-                        F2 hA[8];
-                        float hB[8];
-                        HVALS(iq, hA, hB);
-                        float Hq[3][8];
-#pragma unroll
-                        for (int t = 0; t < 8; t++) {
-                            Hq[0][t] = kind[t] == 1 ? hA[t].x() : 0.f;
-                            Hq[1][t] = kind[t] == 1 ? hA[t].y() : 0.f;
-                            Hq[2][t] = kind[t] == 1 ? hB[t] : 0.f;
-                        }
-#pragma unroll
-                        for (int t = 0; t < 8; t++) {
-                            if (kind[t] == 2) {
-                                const int o = hg_corner(t);
-#pragma unroll
-                                for (int ic = 0; ic < 3; ic++) {
-                                    float Vc[8];
-#pragma unroll
-                                    for (int m = 0; m < 8; m++) {
-                                        const int n = hg_corner(m);
-                                        const int dj = (n & 1) - (o & 1), dk = ((n >> 1) & 1) - ((o >> 1) & 1),
-                                                  dl = (n >> 2) - (o >> 2);
-                                        const float* vp = ic == 0 ? A.vin[0] : ic == 1 ? A.vin[1] : A.vin[2];
-                                        Vc[m] = vp[g.idx(jn + dj, kn + dk, l + dl)];
-                                    }
-                                    const float hv = yc[t] * hg_sum(Vc, iq);
-                                    if (ic == 0) Hq[0][t] = hv;
-                                    else if (ic == 1) Hq[1][t] = hv;
-                                    else Hq[2][t] = hv;
-                                }
-                            }
-                        }
-#pragma unroll
-                        for (int ic = 0; ic < 3; ic++) f[ic] = f[ic] - hg_sum(Hq[ic], iq);
-                    }
-                }
             }
         }
         add_force(q, f);
@@ -1048,7 +838,6 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
 
     // ---------------------------------------------------------------- stream
     // ring: planes L0-1, L0, L0+1; staged: L0+2 in flight
-    constexpr std::true_type path{};
 #pragma unroll 1
     for (int p = -1; p <= 1; p++) {
         fetch(L0 + p);
@@ -1064,14 +853,14 @@ __global__ void __launch_bounds__(NTH, GEOM == GEOM_GENERAL ? 1 : 2) k_interior(
 #pragma unroll 1
     for (int l = L0 - 1; l <= L1; l++) {
         const bool first = l < L0;  // the cell plane below the first node plane
-        cells(l, path);
+        cells(l);
         float nxt[5], nuv[6];
         stat_load(l + 1, nxt);
         if (!first) cp_async_wait_all();
         __syncthreads();  // cell plane l complete, staged plane l+2 landed
         if (!first) store((l + 2) % 3);
         if constexpr (FM) nodes_fm(l, !first);
-        else if (!first) nodes(l, path);
+        else if (!first) nodes(l);
         if (!first) uv_load(l + 1, nuv);
         __syncthreads();  // ring slot l+2 complete, staging and cell slot l-1 free
         if (!first) {

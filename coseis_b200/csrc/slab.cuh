@@ -35,7 +35,11 @@ struct LaySl {
     static constexpr int RAWF = 10;                      // staged plane: u(3) v(3) gam x y z
     static constexpr int RAWSZ = (RAWF * NPL + 3) & ~3;  // floats, float4-aligned end
     static constexpr int NGN = 3;                        // node groups: (u, x), (v, gam), (y, z)
-    static constexpr int NDIR = Lay<GEOM>::NDIR, NQ = Lay<GEOM>::NQ, NGCF = Lay<GEOM>::NGCF;
+    static constexpr int NDIR = Lay<GEOM>::NDIR;
+    // groups per cell: (e11 e22 e33 e23), (e31 e12) as float2, then per reading
+    // node column q, NQ groups: its hourglass sums for the node above and
+    // below, and its divergence brackets
+    static constexpr int NQ = 3, NGCF = 2 + 4 * NQ;
     static constexpr size_t bytes = sizeof(float) * (size_t)RAWSZ + sizeof(float4) * (size_t)(3 * NPL * NGN + NCL * NGCF);
 };
 
@@ -149,7 +153,7 @@ __global__ void __launch_bounds__(SJ * SK, 1) k_slab(StepArgs A) {
     auto cells = [&](int l) {
         const bool valid = cellcol && l >= g.i1cell[2] && l <= g.i2cell[2];
         if (!valid) {
-            zero_cell_fm<NDIR, NQ>(sC, tid, NCL_);
+            zero_cell_fm(sC, tid, NCL_);
             return;
         }
         // one damped axis (classes 1, 2, 4): this cell's g memory is loaded
@@ -298,7 +302,7 @@ __global__ void __launch_bounds__(SJ * SK, 1) k_slab(StepArgs A) {
                 }
             }
         }
-        // fast layout (Lay::NGCF): stress, then per reading node column q the
+        // fast layout (LaySl::NGCF): stress, then per reading node column q the
         // hourglass sums for the node above and below the cell and the
         // divergence brackets
         float4* cw = sC + tid;
