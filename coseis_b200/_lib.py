@@ -157,7 +157,7 @@ def binomial_cost(nt, snapshots):
 
 def trim_memory(device=0):
     """Return the device memory of destroyed handles to the driver now (a
-    helper thread returns it, the last 2 GiB after ten seconds)."""
+    helper thread returns it, the last 2 GiB after a minute without a handle)."""
     _check(load().sord_trim_memory(device))
 
 

@@ -3,6 +3,7 @@
 // (utilities.f90:120-165) and rinvert (utilities.f90:40-49).
 #include <unistd.h>
 
+#include <algorithm>
 #include <chrono>
 #include <condition_variable>
 #include <cstdint>
@@ -226,14 +227,14 @@ void smem_limit(const void* func, int bytes) {
 // (a gradient of 64^3 nodes and 120 kept states, 1.2 GiB: the forward run's
 // allocations 30 ms and the wait in sord_create 4 to 100 ms, now 9 ms for
 // the forward run and 2 ms to create; 1/90 of the device's memory is kept).
-// The rest goes back once no handle has been made for kPoolIdle, or at once
-// by sord_trim_memory.  Returning tens of GB to the driver takes up to
+// The rest goes back once no handle has been made for a minute
+// (SORD_POOL_IDLE seconds), or at once by sord_trim_memory.  Returning tens of GB to the driver takes up to
 // seconds, so both trims run on a helper thread and the destroying call
 // returns at once; the next handle created on that device, and the exit of
 // the process (an atexit handler, registered after the CUDA runtime's own
 // and so run before it), end its wait and wait for a trim under way.
 static constexpr uint64_t kPoolKeep = (uint64_t)2 << 30;
-static constexpr std::chrono::seconds kPoolIdle{10};
+static constexpr int kPoolIdle = 60;  // seconds
 static std::mutex g_mem_m;
 static std::map<int, int> g_live;  // device -> live handles
 struct Trim {
@@ -311,12 +312,14 @@ void mem_detach(int device) {
             std::call_once(at_exit, [] { std::atexit(trim_join_all); });
             Trim& t = g_trim[device];
             t.stop = false;
+            const char* env = getenv("SORD_POOL_IDLE");
+            const std::chrono::seconds idle(env && *env ? std::max(0, atoi(env)) : kPoolIdle);
             try {
-                t.thread = std::thread([device, pool, &t] {
+                t.thread = std::thread([device, pool, idle, &t] {
                     cudaSetDevice(device);
                     cudaMemPoolTrimTo(pool, kPoolKeep);
                     std::unique_lock<std::mutex> lock(t.m);
-                    if (!t.cv.wait_for(lock, kPoolIdle, [&t] { return t.stop; })) pool_release(pool);
+                    if (!t.cv.wait_for(lock, idle, [&t] { return t.stop; })) pool_release(pool);
                 });
                 g_trim_pid = getpid();
             } catch (const std::exception&) {  // no thread to be had

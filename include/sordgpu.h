@@ -153,11 +153,11 @@ int sord_adjoint_backward(sord_handle* h, int nrec, const char* const* files, co
  * pool; when the last handle on a device is destroyed the pool's memory is
  * returned to the driver on a helper thread, so sord_destroy and
  * sord_run_directory return without waiting for it: all but 2 GiB, which the
- * next handle may use, at once, and those when ten seconds have passed
- * without one.  sord_trim_memory with no live handle on `device` returns
- * the pool's unused memory now: call it before allocating the memory
- * elsewhere.  No reference counterpart (the reference frees its arrays
- * at process exit). */
+ * next handle may use, at once, and those when a minute (SORD_POOL_IDLE
+ * seconds, where that is set) has passed without one.  sord_trim_memory with
+ * no live handle on `device` returns the pool's unused memory now: call it
+ * before allocating the memory elsewhere.  No reference counterpart (the
+ * reference frees its arrays at process exit). */
 int sord_trim_memory(int device);
 
 /* After sord_adjoint_backward: the gradients with respect to the position

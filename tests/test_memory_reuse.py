@@ -16,12 +16,13 @@ def handle(path, n):
 
 
 @pytest.mark.gpu
-def test_memory_goes_back_without_a_call(tmp_path, gpu_lib):
+def test_memory_goes_back_without_a_call(tmp_path, monkeypatch, gpu_lib):
     """The fields of a closed handle (1.4 GB) serve the next one, and go back
-    to the driver by themselves when none comes; sord_trim_memory returns
-    them at once."""
+    to the driver by themselves when none comes (within SORD_POOL_IDLE
+    seconds); sord_trim_memory returns them at once."""
     import torch
     from coseis_b200 import _lib
+    monkeypatch.setenv('SORD_POOL_IDLE', '4')
     free = lambda: torch.cuda.mem_get_info()[0]
     handle(str(tmp_path / 'first'), 220).close()  # what a first handle loads stays
     _lib.trim_memory(0)
