@@ -1090,7 +1090,9 @@ static FusedPlan& fused_plan(Solver& s) {
         P->nby = (int)div_up(P->kend - P->kf + 1, FOK);
         const int planes = P->lf1 - P->lf0 + 1, cols = P->nbx * P->nby;
         // the split that takes the fewest plane times: rounds of two blocks
-        // per SM, each block its planes and a prologue of about two.  (An
+        // per SM, as many as are resident on rectilinear and terrain meshes
+        // (one on general meshes, for which the rule has not been tuned), each
+        // block its planes and a prologue of about two.  (An
         // even spread with half a last round, as if blocks did not come in
         // rounds, splits further: 5 % slower on 256 x 256 x 128 nodes in
         // reference order, where the shell's blocks fill the gaps anyway.)

@@ -17,7 +17,7 @@
 // plane, and the force sums that the last cell leaves on its upper plane.
 // A node plane's force reaches the nodes once both of its cells are in, as
 // four corner values per thread, of which one is the thread's own node's.
-// //
+//
 // In the PML shell (MASK: the axes that may be damped in a box) a cell's
 // gradient along a damped axis is that of v, through the g memory; along the
 // others it is that of u, not w (stress.f90:18-131).  Divergence along a
@@ -27,9 +27,10 @@
 // node, the stiffness one, yy hg1 of u, only on nodes outside the PML
 // (acceleration.f90:136-199), so it joins the force at the corner values.
 //
-// Bound by instruction issue (0.77 of the slots in the interior, 0.39-0.55 in
-// the shell, whose blocks wait on the g and p memories).  Against the
-// kernels that evaluated each bracket sum on its own, per launch on a B200:
+// The interior is bound by instruction issue (0.71 of the slots on 203 x 149 x
+// 97 terrain nodes); the shell's classes issue 0.33 to 0.46, their blocks
+// waiting on the g and p memories.  Against the kernels that evaluated each
+// bracket sum on its own, per launch on a B200:
 //   512 x 512 x 256 terrain, 12-node PML  interior 1884 -> 1536 us, shell
 //     classes x 415 -> 391, y 424 -> 327, z 288 -> 224, edges 162 -> 102 us
 //   300 x 150 x 150 rectilinear, 10-node PML  interior 162 -> 134 us, x 65 ->
@@ -54,8 +55,9 @@ struct LayM {
     static constexpr int NS = 5;              // ring slots (node planes), each [(u, gam)][NP], [(v, z)][NP]
     static constexpr int ND = (MASK & 1) + ((MASK >> 1) & 1) + ((MASK >> 2) & 1);  // damped axes
     static constexpr int NSET = 1 + ND;  // force sets: the undamped part, then each damped axis's divergence
-    // buffers of the force values: two save a barrier per plane, one lets
-    // a second block of the edges and corners fit on an SM
+    // buffers of the force values: two save a barrier per plane.  (The edges
+    // and corners have one, 95 KB a block instead of 144; a second block would
+    // fit beside it, but their registers leave room for one only.)
     static constexpr int NB = MASK == 7 ? 1 : 2;
     static constexpr size_t bytes = 16 * (size_t)(NS * 2 * NP + NB * NSET * 3 * NT);
 };
@@ -83,9 +85,12 @@ __global__ void k_statics(Geom g, const float* __restrict__ lam, const float* __
 // MASK 0: tiles of 31 x 7 nodes from (A.jf, A.kf), planes A.lf0..A.lf1,
 // strictly inside the non-PML region.  Otherwise: the boxes A.items.
 // Two cell planes are kept in flight (five ring slots) and the PML memories
-// are read at the start of a plane's work; the edges and corners (MASK 7)
-// take all registers for one block per SM, since their twelve memories spill
-// at two (102 against 137 us at 512 x 512 x 256).
+// are read at the start of a plane's work.  Two blocks per SM leave a thread
+// 128 registers: the interior fits, the classes of one axis spill (20 to 60
+// bytes stored on rectilinear meshes, 120 to 330 on terrain); the edges and
+// corners (MASK 7), whose memories of three axes are 18 values, take 199 to
+// 244 registers for one block per SM (102 us against 137 with two, at 512 x
+// 512 x 256).
 // PLAIN: a folded step without statistics, acceleration output or fault,
 // whose branches are compiled out.
 template <int GEOM, int MASK, bool PLAIN>

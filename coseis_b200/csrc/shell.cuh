@@ -16,7 +16,8 @@
 // start of a plane's work, and the corners come from shared memory, where
 // one kernel for all classes took 164 warp instructions per node with 48
 // loads per PML cell from device memory.  256 x 256 x 128 terrain, 12-node
-// PML: 15.1 -> 12.5 ms for ten steps; the classes also run side by side.
+// PML: 15.1 -> 12.5 ms for ten steps; the classes also run side by side.  At
+// two blocks per SM the classes of one axis spill 150 to 290 bytes a thread.
 #pragma once
 
 template <int GEOM>
