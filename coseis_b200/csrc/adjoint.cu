@@ -1145,9 +1145,14 @@ void adjoint_backward(Solver& s, int nrec, const char* const* files, const float
         cudaStream_t side = nullptr;  // k_adj_step of a run with PML
         cudaEvent_t ev[7] = {};  // rec_done[2], adj_done[2], start, fork, join
         ~Streams() {
+            // after an error the adjoint state that their kernels use may be
+            // freed on the solver's stream, which has not joined them
             for (auto e : ev) if (e) cudaEventDestroy(e);
-            if (as) cudaStreamDestroy(as);
-            if (side) cudaStreamDestroy(side);
+            for (cudaStream_t st : {as, side})
+                if (st) {
+                    cudaStreamSynchronize(st);
+                    cudaStreamDestroy(st);
+                }
         }
     } S;
     SORD_CUDA(cudaStreamCreateWithFlags(&S.as, cudaStreamNonBlocking));
